@@ -189,6 +189,11 @@ psb_status himeno_tb2_launch(MapImpl &m1, MapImpl &m2, GridImpl *in, GridImpl *o
 psb_status generic_tma_launch(MapImpl &m, const GenericDesc &gd, int color, cudaStream_t s,
                               int64_t *launches);
 void generic_note_impl(int impl);
+bool generic_compile_on();
+// The point kernel compiled for the table (k_generic_pt.cu):
+// PSB_ERR_UNSUPPORTED when the map keeps the interpreting kernel.
+psb_status generic_points_launch(MapImpl &m, const GenericDesc &gd, int color, cudaStream_t s,
+                                 int64_t *launches);
 psb_status generic_launch(MapImpl &m, const GenericDesc &d, int color, cudaStream_t s,
                           int64_t *launches);
 psb_status reduce_view(const GridView &v, int type, int op, const Dom3 &dom, double *result,

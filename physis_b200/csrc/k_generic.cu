@@ -111,6 +111,13 @@ psb_status generic_launch(MapImpl &m, const GenericDesc &gd, int color, cudaStre
   dim3 grid((ext[0] + block.x - 1) / block.x, (ext[1] + block.y - 1) / block.y,
             (ext[2] + block.z - 1) / block.z);
   if (grid.y > 65535 || grid.z > 65535) return set_status(PSB_ERR_INVALID);
+  // Compiled for the table where that can be done; the interpreting kernel
+  // below is what runs without a run-time compiler (and what the compiled
+  // forms are tested against).
+  if (rt().impl != PSB_IMPL_PLAIN && rt().impl != PSB_IMPL_GENERIC) {
+    const psb_status st = generic_points_launch(m, gd, color, s, launches);
+    if (st != PSB_ERR_UNSUPPORTED) return st;
+  }
   const GenTable *tab = (const GenTable *)gd.dev;
   switch (desc.accum_type) {
     case PS_FLOAT: k_generic<float><<<grid, block, 0, s>>>(tab, G, d, color); break;

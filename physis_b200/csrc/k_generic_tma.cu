@@ -98,7 +98,7 @@ static int g_last_generic_impl = PSB_IMPL_GENERIC;
 static int g_last_generic_compiled = 0;
 static int g_generic_compile = -1;  // -1: $PHYSIS_B200_GENERIC_COMPILE (default on)
 
-static bool generic_compile_on() {
+bool generic_compile_on() {
   if (g_generic_compile < 0) {
     const char *e = getenv("PHYSIS_B200_GENERIC_COMPILE");
     g_generic_compile = e && e[0] == '0' ? 0 : 1;
