@@ -605,13 +605,14 @@ def run_ours(args):
     hbm, peak_kind = peaks()
     # Compulsory bytes of every update over the device time (GLUPS x B/LUP):
     # the same as per-launch bytes over launch time when every launch is one
-    # step; with two steps per launch (temporal blocking) it is the effective
+    # step; with several steps per launch (temporal blocking) it is the effective
     # bandwidth and may exceed the copy peak.
     achieved = bpl * pts_per_step * args.steps / dev_s / 1e9
     two_sweeps = kname == "himeno" and tune is not None and tune.get("t_depth") == 2
-    two_steps = kname == "diffusion7" and tune is not None and tune.get("t_depth") == 2
+    passes = kname == "diffusion7" and not args.plain and launches < tsteps * args.steps
     kname_traffic = ("k_himeno_tb2" if two_sweeps else "k_himeno_tma") if kname == "himeno" else \
-        ("k_diff7_tb2_f32" + ("_fma" if fma else "")) if two_steps else \
+        ("k_diff7_pipe_%s" % ("f32" if dt == np.float32 else "f64") + ("_fma" if fma else "")) \
+        if passes else \
         "k_generic_tma_f32" if kname == "generic27" else "k_dsl_diffusion7_f32" if kname == "dsl7" \
         else "k_dsl_box27_f32" if kname == "dsl27" else (
         "k_diff7_tma_f32" if dt == np.float32 else "k_diff7_tma_f64") + ("_fma" if fma else "")
@@ -710,7 +711,7 @@ def run_ours(args):
             "avg_launch_us": per_launch_s * 1e6,
             "steps_per_launch": (tsteps * args.steps) / launches,
             "achieved_is": "compulsory bytes per lattice update x updates / device time "
-                           "(effective; with two steps per launch it may exceed the peak)",
+                           "(effective; with several steps per launch it may exceed the peak)",
         },
         "e2e": {"value": e2e_value, "unit": "GLUPS", "h2d_bytes_per_step": int(nbytes),
                 "d2h_bytes_per_step": int(nbytes), "steps": e2e_steps,

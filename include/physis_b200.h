@@ -675,7 +675,8 @@ typedef struct {
   int tile_y;       /* points per CTA in y */
   int z_chunk;      /* planes per CTA work item */
   int stages;       /* pipelined planes in flight */
-  int t_depth;      /* temporal blocking depth (1 = none) */
+  int t_depth;      /* steps per pass (1: single steps; 2: passes of two, for
+                     * a 7-point entry on tile_y 16 of up to four) */
 } psb_tune_config;
 psb_status psb_autotune(int kernel_id, int type, const PSIndex *dims, int force,
                         psb_tune_config *cfg);

@@ -1586,7 +1586,8 @@ psb_status psb_batch_run(psb_batch *b, int mode) {
   legacy_join_in();
   // Periodic members read their input's resident halo.
   for (auto &h : b->hm)
-    if (h.kind == BK_DIFF7P && h.grids[0]->ghost_valid != PSB_BOUNDARY_PERIODIC)
+    if (h.kind == BK_DIFF7P && h.grids[0]->ghost_valid != PSB_BOUNDARY_PERIODIC &&
+        h.grids[0]->ghost_valid != kGhostFaces)
       PSB_CHECK(launch_halo_fill(h.grids[0], PSB_BOUNDARY_PERIODIC, r.stream));
   if (mode == 0 || mode == 1) {
     if (!b->built) {
@@ -1618,10 +1619,10 @@ psb_status psb_batch_run(psb_batch *b, int mode) {
   int64_t lups = 0;
   for (auto &h : b->hm) {
     lups += h.points * h.steps;
-    // Writers keep the output halo of periodic members current.
+    // Writers keep the output halo's faces of periodic members current.
     if (h.kind == BK_DIFF7P) {
-      h.grids[0]->ghost_valid = PSB_BOUNDARY_PERIODIC;
-      h.grids[1]->ghost_valid = PSB_BOUNDARY_PERIODIC;
+      h.grids[0]->ghost_valid = kGhostFaces;
+      h.grids[1]->ghost_valid = kGhostFaces;
     } else {
       h.grids[0]->ghost_valid = h.grids[1]->ghost_valid = PSB_BOUNDARY_NONE;
     }

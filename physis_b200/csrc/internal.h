@@ -22,6 +22,11 @@ namespace psb {
 // Host-side objects
 // ---------------------------------------------------------------------------
 
+// Partial periodic halos that 7-point writers leave: the six faces one cell
+// deep (single steps), or x and y two cells deep with their corners on the
+// grid's own planes (multi-step passes, which wrap z themselves).
+constexpr int kGhostFaces = 100, kGhostXY = 101;
+
 struct GridImpl {
   __PSGrid pub;  // must stay first: handles are cast to __PSGrid*
   union {
@@ -38,7 +43,9 @@ struct GridImpl {
   int64_t pitch = 0, rows = 0, planes = 0;
   int pad_left = 0;           // x cells left of the origin
   int halo = 0;               // y/z halo cells (and minimum x halo)
-  int ghost_valid = PSB_BOUNDARY_NONE;  // which halo content is current
+  // Which halo content is current: a PSB_BOUNDARY_* form over the whole halo
+  // (every depth, edges and corners), or one of the kGhost* states.
+  int ghost_valid = PSB_BOUNDARY_NONE;
   bool user_type = false;
   __PSGrid_devFreeFunc user_free = nullptr;
   uint32_t magic = 0x50534232u;
@@ -179,10 +186,16 @@ psb_status diffusion7_launch(MapImpl &m, const psb_tune_config &cfg, cudaStream_
                              int64_t *launches);
 psb_status himeno_launch(MapImpl &m, const psb_tune_config &cfg, cudaStream_t s,
                          int64_t *launches);
-// Two steps of a clamped float 7-point map over a whole pitched grid in one
-// launch (temporal blocking): reads in, writes out.
-psb_status diffusion7_tb2_launch(MapImpl &m, GridImpl *in, GridImpl *out, int zchunk,
-                                 cudaStream_t s, int64_t *launches);
+// ns steps of a 7-point map over whole pitched grids in one pass
+// (k_diff7_pipe.cu): r rows a thread, 2^xl_shift lanes a row.
+struct PipeConfig {
+  int ns, r, threads, xl_shift, zchunk, stages;
+};
+psb_status diff7_pipe_launch(MapImpl &m, GridImpl *in, GridImpl *out, const PipeConfig &cfg,
+                             cudaStream_t s, int64_t *launches);
+// The shape of passes of ns steps over grids of extents n, with its estimated
+// time in SM cycles (< 0: no shape fits).
+PipeConfig diff7_pipe_choose(int ns, bool dbl, bool per, bool fast, const int *n, double *cost);
 bool himeno_tb2_pair(MapImpl **ms, int n);
 psb_status himeno_tb2_launch(MapImpl &m1, MapImpl &m2, GridImpl *in, GridImpl *out,
                              int zchunk, cudaStream_t s, int64_t *launches);
@@ -208,6 +221,8 @@ void maps_forget_grid(const GridImpl *g);
 
 // Autotuning.
 psb_tune_config default_config(int kernel, int type, const int *n);
+// The table's entry for a shape, if it has one.
+bool tune_find(int kernel, int type, const int *n, psb_tune_config *cfg);
 psb_status tune_lookup(int kernel, int type, const int *n, psb_tune_config *cfg);
 // Batched members are tuned per (kernel kind, element type, size bucket):
 // each extent rounded up to a power of two. Their entries live in the same

@@ -189,7 +189,8 @@ static psb_status check_map(const MapImpl &m, bool writes = true) {
 psb_status prepare_ghosts(MapImpl &m) {
   if (m.kernel_id != PSB_KERNEL_DIFFUSION7_PERIODIC) return PSB_OK;
   GridImpl *in = m.grids[0];
-  if (in->layout == PSB_LAYOUT_PITCHED && in->ghost_valid != PSB_BOUNDARY_PERIODIC)
+  if (in->layout == PSB_LAYOUT_PITCHED && in->ghost_valid != PSB_BOUNDARY_PERIODIC &&
+      in->ghost_valid != kGhostFaces)
     return launch_halo_fill(in, PSB_BOUNDARY_PERIODIC, rt().stream);
   return PSB_OK;
 }
@@ -214,13 +215,16 @@ psb_status launch_map(MapImpl &m, int color, int64_t *launches) {
     GridImpl *o = m.grids[1];
     if (m.kernel_id != PSB_KERNEL_DIFFUSION7_PERIODIC && o->layout == PSB_LAYOUT_PITCHED)
       o->ghost_valid = PSB_BOUNDARY_NONE;
-    // Periodic writers keep the output halo current (images), so a valid
-    // halo stays valid; an incomplete domain cannot make it valid.
+    // Periodic writers keep the faces of the output halo current (images one
+    // cell deep), so valid faces stay valid; an incomplete domain cannot make
+    // them valid.
     if (m.kernel_id == PSB_KERNEL_DIFFUSION7_PERIODIC && o->layout == PSB_LAYOUT_PITCHED) {
       bool full = true;
       for (int i = 0; i < 3; i++)
         if (m.dom.local_min[i] != 0 || m.dom.local_max[i] != o->pub.dim[i]) full = false;
-      if (full) o->ghost_valid = PSB_BOUNDARY_PERIODIC;
+      const bool faces =
+          o->ghost_valid == PSB_BOUNDARY_PERIODIC || o->ghost_valid == kGhostFaces;
+      o->ghost_valid = full || faces ? kGhostFaces : PSB_BOUNDARY_NONE;
     }
   } else if (const psb_compiled_stencil *cd = compiled_of(m.kernel_id)) {
     GridImpl *views[PSB_MAX_VIEWS];
@@ -306,24 +310,26 @@ void maps_forget_grid(const GridImpl *g) {
   }
 }
 
-// The pattern temporal blocking applies to: PSStencilRun(m1, m2, iter) with
-// m1: A -> B and m2: B -> A the same clamped float 7-point map over the
-// whole of two pitched grids.
-static bool tb2_pair(MapImpl **ms, int n) {
+// The pattern that passes of several steps apply to: PSStencilRun(m1, m2,
+// iter) with m1: A -> B and m2: B -> A the same 7-point map (clamped or
+// periodic) over the whole of two pitched grids of at least four points a
+// side (a periodic pass wraps up to two).
+static bool pipe_pair(MapImpl **ms, int n) {
   if (n != 2) return false;
   const MapImpl &a = *ms[0], &b = *ms[1];
-  if (a.kernel_id != PSB_KERNEL_DIFFUSION7 || b.kernel_id != PSB_KERNEL_DIFFUSION7) return false;
-  if (a.color != -1 || b.color != -1 || a.nparams != 7 || b.nparams != 7) return false;
+  if (a.kernel_id != PSB_KERNEL_DIFFUSION7 && a.kernel_id != PSB_KERNEL_DIFFUSION7_PERIODIC)
+    return false;
+  if (b.kernel_id != a.kernel_id || a.color != -1 || b.color != -1) return false;
   for (int i = 0; i < 7; i++)
     if (a.params[i] != b.params[i]) return false;
   GridImpl *A = a.grids[0], *B = a.grids[1];
   if (b.grids[0] != B || b.grids[1] != A || A == B) return false;
   for (GridImpl *g : {A, B}) {
-    if (g->layout != PSB_LAYOUT_PITCHED || g->type != PS_FLOAT || g->pub.num_dims != 3 ||
-        !tma_eligible(g))
+    if (g->layout != PSB_LAYOUT_PITCHED || g->type != A->type || !tma_eligible(g) ||
+        (g->type != PS_FLOAT && g->type != PS_DOUBLE))
       return false;
     for (int i = 0; i < 3; i++)
-      if (g->pub.dim[i] != A->pub.dim[i]) return false;
+      if (g->pub.dim[i] != A->pub.dim[i] || g->pub.dim[i] < 4) return false;
   }
   for (const MapImpl *m : {&a, &b})
     for (int i = 0; i < 3; i++)
@@ -331,19 +337,84 @@ static bool tb2_pair(MapImpl **ms, int n) {
   return true;
 }
 
-// iter pairs as F two-step launches (F the largest even number below iter)
-// alternating A -> B and B -> A, then the remaining one or two pairs
-// unfused: both grids end exactly as after the unfused run (A the last
-// step, B the one before it).
-static psb_status run_tb2(MapImpl **ms, int iter, int zchunk, int64_t *launches) {
+// How a run of `iter` pairs is cut: passes of four and two steps and single
+// steps, alternating A -> B and B -> A. Both grids have to end as after
+// single steps (A the last step, B the one before it), so the last step is a
+// single one from B, and the passes before it, 2 iter - 1 steps, are an odd
+// number of launches (three singles where one does not come out odd).
+struct PipePlan {
+  PipeConfig four, two;
+  int fours = 0, twos = 0, singles = 0;
+};
+
+// False: the run keeps single steps. A tune entry of a clamped float shape
+// decides: t_depth 1 keeps single steps, t_depth 2 two-step passes only, and
+// t_depth 2 on tile_y 16 whatever passes are estimated fastest, which is also
+// the rule without an entry and for the other kinds (the tuner records only
+// single-step shapes for them).
+static bool pipe_plan(MapImpl **ms, int iter, PipePlan *plan) {
+  const Runtime &r = rt();
+  const GridImpl *A = ms[0]->grids[0];
+  const int *n = A->pub.dim;
+  const bool dbl = A->type == PS_DOUBLE, fast = r.fp_mode == PSB_FP_FMA;
+  const bool per = ms[0]->kernel_id == PSB_KERNEL_DIFFUSION7_PERIODIC;
+  bool free_choice = true;
+  psb_tune_config cfg;
+  if (tune_find(ms[0]->kernel_id, dbl ? PS_DOUBLE : PS_FLOAT, n, &cfg) && !per && !dbl) {
+    if (cfg.t_depth != 2) return false;
+    free_choice = cfg.tile_y == 16;
+  }
+  const int steps = 2 * iter - 1;  // before the last one
+  double t4 = -1, t2 = -1;
+  if (free_choice && !per) plan->four = diff7_pipe_choose(4, dbl, per, fast, n, &t4);
+  plan->two = diff7_pipe_choose(2, dbl, per, fast, n, &t2);
+  if (t2 < 0) return false;
+  if (!free_choice) {
+    plan->twos = (iter - 1) & ~1;
+    plan->singles = steps - 2 * plan->twos;
+    return plan->twos > 0;
+  }
+  // A single step: its launch, and its bytes at about the L2 rate while both
+  // grids fit, the HBM rate beyond (cycles).
+  const double bytes = 2.0 * A->pub.elm_size * A->pub.num_elms;
+  const double t1 = 6000 + bytes / (bytes < 100e6 ? 2000.0 : 3000.0);
+  double best = t1 * steps;
+  for (int c = 1; c <= 3 && c <= steps; c += 2)
+    for (int b = 0; 2 * b <= steps - c; b++) {
+      const int left = steps - c - 2 * b;
+      if (left % 4 || (left && t4 < 0)) continue;
+      const int a = left / 4;
+      if ((a + b + c) % 2 == 0) continue;
+      const double t = a * t4 + b * t2 + c * t1;
+      if (t < best) {
+        best = t;
+        plan->fours = a;
+        plan->twos = b;
+        plan->singles = c;
+      }
+    }
+  return plan->fours + plan->twos > 0;
+}
+
+static psb_status run_pipe(MapImpl **ms, const PipePlan &plan, int64_t *launches) {
   Runtime &r = rt();
-  GridImpl *A = ms[0]->grids[0], *B = ms[0]->grids[1];
-  const int F = (iter - 1) & ~1;
-  for (int f = 0; f < F; f++)
-    PSB_CHECK(diffusion7_tb2_launch(*ms[0], f & 1 ? B : A, f & 1 ? A : B, zchunk, r.stream,
-                                    launches));
-  A->ghost_valid = B->ghost_valid = PSB_BOUNDARY_NONE;
-  for (int it = F; it < iter; it++) PSB_CHECK(launch_iteration(ms, 2, launches));
+  const bool per = ms[0]->kernel_id == PSB_KERNEL_DIFFUSION7_PERIODIC;
+  GridImpl *g[2] = {ms[0]->grids[0], ms[0]->grids[1]};
+  int at = 0;  // the grid that holds the state
+  for (int i = 0; i < plan.fours + plan.twos; i++) {
+    GridImpl *in = g[at], *out = g[at ^ 1];
+    if (per && in->ghost_valid != PSB_BOUNDARY_PERIODIC && in->ghost_valid != kGhostXY)
+      PSB_CHECK(launch_halo_fill(in, PSB_BOUNDARY_PERIODIC, r.stream));
+    PSB_CHECK(diff7_pipe_launch(*ms[0], in, out, i < plan.fours ? plan.four : plan.two, r.stream,
+                                launches));
+    out->ghost_valid = per ? kGhostXY : PSB_BOUNDARY_NONE;
+    at ^= 1;
+  }
+  for (int i = 0; i <= plan.singles; i++) {
+    PSB_CHECK(prepare_ghosts(*ms[at]));
+    PSB_CHECK(launch_map(*ms[at], -1, launches));
+    at ^= 1;
+  }
   return PSB_OK;
 }
 
@@ -364,23 +435,23 @@ static psb_status run_maps(MapImpl **ms, int n, int iter) {
   Runtime &r = rt();
   if (iter <= 0) return PSB_OK;
   for (int i = 0; i < n; i++) PSB_CHECK(check_map(*ms[i]));
-  for (int i = 0; i < n; i++) PSB_CHECK(prepare_ghosts(*ms[i]));
+  const bool pipe = r.impl != PSB_IMPL_PLAIN && r.impl != PSB_IMPL_GENERIC && iter >= 2 &&
+                    pipe_pair(ms, n);
+  for (int i = 0; i < n && !pipe; i++) PSB_CHECK(prepare_ghosts(*ms[i]));
   int64_t launches = 0;
   legacy_join_in();
   PSB_TRY(cudaEventRecord(r.ev_start, r.stream));
-  if (r.impl != PSB_IMPL_PLAIN && r.impl != PSB_IMPL_GENERIC && tb2_pair(ms, n)) {
-    psb_tune_config cfg;
-    const int *dims = ms[0]->grids[0]->pub.dim;
-    tune_lookup(PSB_KERNEL_DIFFUSION7, PS_FLOAT, dims, &cfg);
-    if (cfg.t_depth == 2) {
-      PSB_CHECK(run_tb2(ms, iter, cfg.z_chunk, &launches));
-      PSB_TRY(cudaEventRecord(r.ev_stop, r.stream));
-      legacy_join_out();
-      r.last_launches = launches;
-      r.last_timed = true;
-      return PSB_OK;
-    }
+  PipePlan plan;
+  if (pipe && pipe_plan(ms, iter, &plan)) {
+    PSB_CHECK(run_pipe(ms, plan, &launches));
+    PSB_TRY(cudaEventRecord(r.ev_stop, r.stream));
+    legacy_join_out();
+    r.last_launches = launches;
+    r.last_timed = true;
+    return PSB_OK;
   }
+  // Single steps read the halos prepared here.
+  for (int i = 0; i < n && pipe; i++) PSB_CHECK(prepare_ghosts(*ms[i]));
   if (r.impl != PSB_IMPL_PLAIN && r.impl != PSB_IMPL_GENERIC && himeno_tb2_pair(ms, n) &&
       iter >= 3) {
     psb_tune_config cfg;

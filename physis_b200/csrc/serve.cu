@@ -462,7 +462,7 @@ static psb_status run_round(psb_server *S, std::vector<SReq *> &finished) {
     for (int k = 0; k < 4; k++) q->res[k] = res[4 * i + k];
     q->residual = residual_of(q->res);
     if (q->kind == BK_DIFF7P)
-      for (int k = 0; k < 2; k++) q->h.grids[k]->ghost_valid = PSB_BOUNDARY_PERIODIC;
+      for (int k = 0; k < 2; k++) q->h.grids[k]->ghost_valid = kGhostFaces;
   }
   {
     std::lock_guard<std::mutex> lk(S->mu);

@@ -171,11 +171,16 @@ void batch_tune_store(int kind, const int *n, const psb_tune_config &cfg) {
 
 void tune_save() { save_cache(); }
 
-psb_status tune_lookup(int kernel, int type, const int *n, psb_tune_config *cfg) {
+bool tune_find(int kernel, int type, const int *n, psb_tune_config *cfg) {
   load_cache();
-  TuneKey k{kernel, type, n[0], n[1], n[2]};
-  auto it = rt().tune.find(k);
-  *cfg = it != rt().tune.end() ? it->second : default_config(kernel, type, n);
+  auto it = rt().tune.find(TuneKey{kernel, type, n[0], n[1], n[2]});
+  if (it == rt().tune.end()) return false;
+  *cfg = it->second;
+  return true;
+}
+
+psb_status tune_lookup(int kernel, int type, const int *n, psb_tune_config *cfg) {
+  if (!tune_find(kernel, type, n, cfg)) *cfg = default_config(kernel, type, n);
   return PSB_OK;
 }
 
@@ -206,6 +211,16 @@ static double time_config(MapImpl &m, const psb_tune_config &cfg, int reps) {
   cudaEventCreate(&b);
   double best = -1;
   int64_t launches = 0;
+  // A 7-point entry with t_depth 2 runs passes of two steps, or on tile_y 16
+  // passes of four where the rule has a shape for them.
+  PipeConfig pass{};
+  if (m.kernel_id != PSB_KERNEL_HIMENO19 && cfg.t_depth == 2) {
+    double cost = -1;
+    const int *n = m.grids[0]->pub.dim;
+    if (cfg.tile_y == 16) pass = diff7_pipe_choose(4, false, false, r.fp_mode == PSB_FP_FMA, n, &cost);
+    if (cost < 0) pass = diff7_pipe_choose(2, false, false, r.fp_mode == PSB_FP_FMA, n, &cost);
+    if (cost < 0) return -1;
+  }
   for (int round = 0; round < 4; round++) {
     cudaEventRecord(a, r.stream);
     for (int i = 0; i < reps; i++) {
@@ -216,9 +231,9 @@ static double time_config(MapImpl &m, const psb_tune_config &cfg, int reps) {
                                                   r.stream, &launches)
                               : himeno_launch(m, cfg, r.stream, &launches);
       else
-        st = cfg.t_depth == 2 ? diffusion7_tb2_launch(m, m.grids[0], m.grids[1], cfg.z_chunk,
-                                                      r.stream, &launches)
-                              : diffusion7_launch(m, cfg, r.stream, &launches);
+        st = cfg.t_depth == 2
+                 ? diff7_pipe_launch(m, m.grids[0], m.grids[1], pass, r.stream, &launches)
+                 : diffusion7_launch(m, cfg, r.stream, &launches);
       if (st != PSB_OK) {
         cudaEventDestroy(a);
         cudaEventDestroy(b);
@@ -233,7 +248,7 @@ static double time_config(MapImpl &m, const psb_tune_config &cfg, int reps) {
     }
     float ms = 0;
     cudaEventElapsedTime(&ms, a, b);
-    ms /= cfg.t_depth == 2 ? 2 : 1;  // per step
+    ms /= pass.ns ? pass.ns : cfg.t_depth == 2 ? 2 : 1;  // per step
     if (round > 0 && (best < 0 || ms / reps < best)) best = ms / reps;  // round 0 warms up
   }
   cudaEventDestroy(a);
@@ -341,17 +356,17 @@ psb_status psb_autotune(int kernel_id, int type, const PSIndex *dims, int force,
           c.t_depth = 1;
           cands.push_back(c);
         }
-  // Temporal blocking (two steps per launch; clamped float 7-point only).
-  // Its tile fields are a valid single-step configuration too, for maps run
-  // alone.
-  if (kernel_id == PSB_KERNEL_DIFFUSION7 && type == PS_FLOAT)
-    for (int zc : {32, 64, 128}) {
-      if (zc > dims[2] * 2) continue;
+  // Passes of several steps (clamped float 7-point): the rule's (tile_y 16)
+  // and two-step passes only (tile_y 8). The fields are a valid single-step
+  // configuration too, for maps run alone.
+  if (kernel_id == PSB_KERNEL_DIFFUSION7 && type == PS_FLOAT && dims[0] >= 4 && dims[1] >= 4 &&
+      dims[2] >= 4)
+    for (int ty : {16, 8}) {
       psb_tune_config c;
       c.impl = PSB_IMPL_TMA;
       c.tile_x = 128;
-      c.tile_y = 8;
-      c.z_chunk = zc;
+      c.tile_y = ty;
+      c.z_chunk = 32;
       c.stages = 6;
       c.t_depth = 2;
       cands.push_back(c);
