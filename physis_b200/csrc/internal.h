@@ -197,6 +197,7 @@ psb_status diff7_pipe_launch(MapImpl &m, GridImpl *in, GridImpl *out, const Pipe
 // time in SM cycles (< 0: no shape fits).
 PipeConfig diff7_pipe_choose(int ns, bool dbl, bool per, bool fast, const int *n, double *cost);
 bool himeno_tb2_pair(MapImpl **ms, int n);
+int himeno_tb2_chunk(const __PSDomain &dom);  // z chunk of the pass over a domain
 psb_status himeno_tb2_launch(MapImpl &m1, MapImpl &m2, GridImpl *in, GridImpl *out,
                              int zchunk, cudaStream_t s, int64_t *launches);
 psb_status generic_tma_launch(MapImpl &m, const GenericDesc &gd, int color, cudaStream_t s,

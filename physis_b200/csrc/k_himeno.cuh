@@ -40,6 +40,44 @@ __device__ __forceinline__ float himeno_point(const float *co, float pc, float p
   return xadd(pc, xmul(omega, ss));
 }
 
+// The pressure values around a thread's four x points, from planes z-1, z and
+// z+1 in shared memory (o: 16-byte aligned offset of the first point, BX: row
+// length, a multiple of 4): the rows the 19 points touch, each as one 16-byte
+// load, with the two values beside it where x neighbours are read (element
+// 1 + v is point v). Scalar loads of the same values, four floats apart from
+// lane to lane, meet four-way bank conflicts and made shared memory the bound
+// of every Himeno kernel: two sweeps at 257x257x513 took 524 us with them.
+struct HimenoRows {
+  float c[6], cn[6], cs[6], p[6], m[6];  // z: y, y-1, y+1; z+1 and z-1: y
+  Vec16<float> pn, ps, mn, ms;           // z+1 and z-1: y-1, y+1
+
+  static __device__ __forceinline__ void row6(const float *q, float (&e)[6]) {
+    const Vec16<float> a = lds16(q);
+    e[0] = q[-1];
+#pragma unroll
+    for (int v = 0; v < 4; v++) e[1 + v] = a.v[v];
+    e[5] = q[4];
+  }
+  __device__ __forceinline__ void load(const float *qm, const float *qc, const float *qp, int o,
+                                       int BX) {
+    row6(qc + o, c);
+    row6(qc + o - BX, cn);
+    row6(qc + o + BX, cs);
+    row6(qp + o, p);
+    row6(qm + o, m);
+    pn = lds16(qp + o - BX);
+    ps = lds16(qp + o + BX);
+    mn = lds16(qm + o - BX);
+    ms = lds16(qm + o + BX);
+  }
+  // Point v with its coefficients (himeno_point).
+  __device__ __forceinline__ float point(const float *co, int v, float omega, float *ss) const {
+    return himeno_point(co, c[1 + v], c[2 + v], c[v], cs[1 + v], cn[1 + v], p[1 + v], m[1 + v],
+                        ps.v[v], pn.v[v], ms.v[v], mn.v[v], cs[2 + v], cn[2 + v], cs[v], cn[v],
+                        p[2 + v], m[2 + v], p[v], m[v], omega, ss);
+  }
+};
+
 struct HimenoGeom {
   int ax0, ay0, az0;
   int tiles_x, tiles_y, zchunk, stages, bx, by, stage_bytes, x_base;
@@ -121,17 +159,15 @@ __device__ __forceinline__ bool himeno_consume(const Ring &R, RingPos &p, float 
     const float *qm = plane_ptr(pm.slot), *qc = plane_ptr(pc.slot), *qp = plane_ptr(pp.slot);
     if (row_in) {
       float outv[V];
+      HimenoRows h;
+      h.load(qm, qc, qp, rc, BX);
 #pragma unroll
       for (int v = 0; v < V; v++) {
-        const int o = rc + v;
         float c[12];
 #pragma unroll
         for (int i = 0; i < 12; i++) c[i] = co[i][v];
         float ss;
-        outv[v] = himeno_point(c, qc[o], qc[o + 1], qc[o - 1], qc[o + BX], qc[o - BX], qp[o],
-                               qm[o], qp[o + BX], qp[o - BX], qm[o + BX], qm[o - BX],
-                               qc[o + 1 + BX], qc[o + 1 - BX], qc[o - 1 + BX], qc[o - 1 - BX],
-                               qp[o + 1], qm[o + 1], qp[o - 1], qm[o - 1], omega, &ss);
+        outv[v] = h.point(c, v, omega, &ss);
         if (xg0 + v >= d.lo[0] && xg0 + v < d.hi[0]) acc += (double)ss * (double)ss;
       }
       float *dst = pout + off;
@@ -233,17 +269,15 @@ __device__ __forceinline__ bool himeno_consume_staged(const Ring &R, RingPos &p,
       for (int i = 0; i < 12; i++)
         co[i] = lds16(reinterpret_cast<const float *>(cs + i * tile_bytes));
       float outv[V];
+      HimenoRows h;
+      h.load(qm, qc, qp, rc, BX);
 #pragma unroll
       for (int v = 0; v < V; v++) {
-        const int o = rc + v;
         float c[12];
 #pragma unroll
         for (int i = 0; i < 12; i++) c[i] = co[i].v[v];
         float ss;
-        outv[v] = himeno_point(c, qc[o], qc[o + 1], qc[o - 1], qc[o + BX], qc[o - BX], qp[o],
-                               qm[o], qp[o + BX], qp[o - BX], qm[o + BX], qm[o - BX],
-                               qc[o + 1 + BX], qc[o + 1 - BX], qc[o - 1 + BX], qc[o - 1 - BX],
-                               qp[o + 1], qm[o + 1], qp[o - 1], qm[o - 1], omega, &ss);
+        outv[v] = h.point(c, v, omega, &ss);
         if (xg0 + v >= d.lo[0] && xg0 + v < d.hi[0]) acc += (double)ss * (double)ss;
       }
       float *dst = pout + off;

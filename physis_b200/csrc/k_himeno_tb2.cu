@@ -194,6 +194,29 @@ bool himeno_tb2_pair(MapImpl **ms, int n) {
   return true;
 }
 
+// The chunk length with the shortest walk: every SM's CTA walks its share of
+// the items one after the other, zc output planes and about 3.5 more for the
+// halo each.
+int himeno_tb2_chunk(const __PSDomain &dom) {
+  const int xb = dom.local_min[0] / kHtV * kHtV;
+  const int nz = dom.local_max[2] - dom.local_min[2];
+  const int64_t tiles = (int64_t)((dom.local_max[0] - xb + kHtTX - 1) / kHtTX) *
+                        ((dom.local_max[1] - dom.local_min[1] + kHtTY - 1) / kHtTY);
+  int best = std::max(nz, 1);
+  double best_cost = -1;
+  for (int nc = 1; nc <= nz && nc <= 256; nc++) {
+    const int zc = (nz + nc - 1) / nc;
+    if (zc < 4 && nc > 1) break;
+    const int64_t items = tiles * ((nz + zc - 1) / zc);
+    const double cost = (double)((items + rt().sm_count - 1) / rt().sm_count) * (zc + 3.5);
+    if (best_cost < 0 || cost < best_cost) {
+      best = zc;
+      best_cost = cost;
+    }
+  }
+  return best;
+}
+
 static psb_status ht_residual(MapImpl &m, int nblocks, Residual *r) {
   *r = Residual{nullptr, m.d_ticket, m.d_counter, m.d_history, m.residual_len};
   if (m.residual_len <= 0) return PSB_OK;

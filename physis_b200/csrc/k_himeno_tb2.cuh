@@ -191,6 +191,8 @@ __device__ __forceinline__ bool ht_stage1_tile(const HtRings &R, RingPos &p1, Ri
 #pragma unroll
       for (int f = 0; f < 12; f++)
         co[f] = lds16(reinterpret_cast<const float *>(cs + f * kHtField) + cofs);
+      HimenoRows h;
+      h.load(qm, qc, qp, pofs, kHtBX);
 #pragma unroll
       for (int v = 0; v < kHtV; v++) {
         const int x = xg + v;
@@ -198,9 +200,9 @@ __device__ __forceinline__ bool ht_stage1_tile(const HtRings &R, RingPos &p1, Ri
 #pragma unroll
         for (int f = 0; f < 12; f++) c[f] = co[f].v[v];
         float ss;
-        const float r = ht_point(c, qm, qc, qp, pofs + v, omega, &ss);
+        const float r = h.point(c, v, omega, &ss);
         const bool in = z_in && row_in && x >= d.lo[0] && x < d.hi[0];
-        outv[v] = in ? r : qc[pofs + v];
+        outv[v] = in ? r : h.c[1 + v];
         if (acc_on && in && z_own && row_own) a += (double)ss * (double)ss;
       }
     }
@@ -280,13 +282,15 @@ __device__ __forceinline__ bool ht_stage2_tile(const HtRings &R, RingPos &p2, Ri
 #pragma unroll
         for (int f = 0; f < 12; f++)
           co[f] = lds16(reinterpret_cast<const float *>(cs + f * kHtField) + ofs);
+        HimenoRows h;
+        h.load(qm, qc, qp, ofs, kHtBX);
 #pragma unroll
         for (int v = 0; v < kHtV; v++) {
           float c[12];
 #pragma unroll
           for (int f = 0; f < 12; f++) c[f] = co[f].v[v];
           float ss;
-          outv[v] = ht_point(c, qm, qc, qp, ofs + v, omega, &ss);
+          outv[v] = h.point(c, v, omega, &ss);
           if (acc_on && xg + v >= d.lo[0] && xg + v < d.hi[0]) a += (double)ss * (double)ss;
         }
       }
