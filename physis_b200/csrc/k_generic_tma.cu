@@ -166,14 +166,106 @@ static std::string gt_jit_source(const GtTable &tab, bool dbl, bool fma, std::st
   return src;
 }
 
+// The plane-by-plane form (gt_body_planes) needs a packed table whose terms
+// come in plane order over two or three planes, and pays from eight terms on.
+// Float at 512^3, this form against the window form: 27 equal coefficients
+// 239 us against 464 (FMA mode 235 against 400), 27 distinct ones 328 against
+// 464; a 7-term star 212 against 205; a 13-term star over five planes, whose
+// running sums leave too few registers, 272 against 243.
+static bool gt_plane_form(const GtTable &tab, const GtGeom &geo) {
+  if (!tab.simple || tab.nterms < 8 || geo.window < 2 || geo.window > 3) return false;
+  for (int t = 1; t < tab.nterms; t++)
+    if ((tab.word[t] & 7) < (tab.word[t - 1] & 7)) return false;
+  return true;
+}
+
+// Source of the plane-by-plane form. Row offsets of the words are split back
+// into grid and dy (plane_elems, bx); equal coefficients are read once, so
+// that the compiler shares their products.
+static std::string gt_jit_plane_source(const GtTable &tab, const GtGeom &geo, bool dbl, bool fma,
+                                       std::string *key) {
+  const char *T = dbl ? "double" : "float";
+  struct Row {
+    bool used = false, p2 = false, p1 = false, n1 = false, n2 = false;
+  };
+  Row rows[kGtMaxGrids][kGtVY + 2 * kGtR];
+  std::vector<int> grid(tab.nterms), dy(tab.nterms), cls(tab.nterms), uses(tab.nterms, 0);
+  std::string k = std::string(T) + (fma ? ":zf:" : ":z:") + std::to_string(geo.window) + ":";
+  for (int t = 0; t < tab.nterms; t++) {
+    const int w = tab.word[t], off = w >> 10, dx = ((w >> 3) & 7) - 2;
+    // off = grid * plane_elems + dy * bx with |dy| <= 2.
+    const int g = (off + 2 * geo.bx) / geo.plane_elems;
+    grid[t] = g;
+    dy[t] = (off - g * geo.plane_elems) / geo.bx;
+    cls[t] = t;
+    for (int u = 0; u < t; u++)
+      if (memcmp(&tab.coef[u], &tab.coef[t], sizeof(double)) == 0) {
+        cls[t] = u;
+        break;
+      }
+    uses[cls[t]]++;
+    for (int r = 0; r < kGtVY; r++) {
+      Row &q = rows[g][kGtR + r + dy[t]];
+      q.used = true;
+      q.p2 = q.p2 || dx == -2;
+      q.p1 = q.p1 || dx == -1 || dx == -2;
+      q.n1 = q.n1 || dx == 1 || dx == 2;
+      q.n2 = q.n2 || dx == 2;
+    }
+    k += std::to_string(w & 1023) + "." + std::to_string(g) + "." + std::to_string(dy[t]) + "." +
+         std::to_string(cls[t]) + ",";
+  }
+  *key = "k_generic_tma:" + k + "vy" + std::to_string(kGtVY);
+  auto b = [](bool v) { return std::string(v ? "true" : "false"); };
+  std::string body;
+  for (int g = 0; g < kGtMaxGrids; g++) {
+    bool any = false;
+    for (const Row &q : rows[g]) any = any || q.used;
+    if (!any) continue;
+    const std::string gs = std::to_string(g);
+    body += "    GtRow<T> q" + gs + "[kGtVY + 2 * kGtR];\n";
+    for (int y = 0; y < kGtVY + 2 * kGtR; y++) {
+      const Row &q = rows[g][y];
+      if (q.used)
+        body += "    gt_row_ext<T, " + b(q.p2) + ", " + b(q.p1) + ", " + b(q.n1) + ", " + b(q.n2) +
+                ">(p + " + gs + " * plane_elems + (" + std::to_string(y - kGtR) + ") * bx, lane, q" +
+                gs + "[" + std::to_string(y) + "]);\n";
+    }
+  }
+  for (int t = 0; t < tab.nterms; t++)
+    if (cls[t] == t)
+      body += "    const T c" + std::to_string(t) + " = gt_coef(tab, " + std::to_string(t) +
+              ", T());\n    (void)c" + std::to_string(t) + ";\n";
+  for (int t = 0; t < tab.nterms; t++) {
+    const int w = tab.word[t];
+    body += "    gt_plane_term<T, " + std::to_string(dy[t]) + ", " + std::to_string((w >> 3) & 7) +
+            ", " + b((w >> 7) & 1) + ", " + b(t == 0) + ", " + b(fma) + ", " +
+            b(uses[cls[t]] > 1) + ">(q" +
+            std::to_string(grid[t]) + ", c" + std::to_string(cls[t]) + ", acc[" +
+            std::to_string((geo.window - (w & 7)) % geo.window) + "]);\n";
+  }
+  return "#include \"k_generic_tma.cuh\"\nnamespace psb {\nstruct GtPlaneProg {\n"
+         "  static constexpr int kWindow = " + std::to_string(geo.window) +
+         ";\n  template <typename T>\n"
+         "  static __device__ __forceinline__ void plane(const GtTable &tab, const T *p, int bx, "
+         "int plane_elems, int lane, GtBlk<T> *acc) {\n" +
+         body + "  }\n};\n}  // namespace psb\n" +
+         "extern \"C\" __global__ void __launch_bounds__(psb::kGtThreads, 3) "
+         "psb_generic_tma_compiled(const __grid_constant__ psb::GtMaps maps, "
+         "const __grid_constant__ psb::GtTable tab, psb::GridView out, psb::Dom3 d, "
+         "const __grid_constant__ psb::GtGeom geo, int *err) {\n  psb::gt_body_planes<" +
+         T + ", psb::GtPlaneProg>(maps, tab, out, d, geo, err);\n}\n";
+}
+
 // The compiled kernel of a table, or nullptr (the interpreting kernel
 // runs). Never compiles while the stream is being captured: the first
 // iteration of every run is eager, so a captured one finds its kernel cached.
-static CUfunction gt_jit(const GtTable &tab, bool dbl, bool fma, cudaStream_t s,
-                         size_t smem_optin) {
+static CUfunction gt_jit(const GtTable &tab, const GtGeom &geo, bool dbl, bool fma,
+                         cudaStream_t s, size_t smem_optin) {
   if (!generic_compile_on()) return nullptr;
   std::string key;
-  const std::string src = gt_jit_source(tab, dbl, fma, &key);
+  const std::string src = gt_plane_form(tab, geo) ? gt_jit_plane_source(tab, geo, dbl, fma, &key)
+                                             : gt_jit_source(tab, dbl, fma, &key);
   CUfunction fn = nullptr;
   cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
   if (cudaStreamIsCapturing(s, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone)
@@ -295,7 +387,7 @@ static psb_status gt_launch(MapImpl &m, const psb_generic_stencil &desc, const G
     if (p.mode[i] != PSB_BOUNDARY_NONE && g->ghost_valid != p.mode[i])
       PSB_CHECK(launch_halo_fill(g, p.mode[i], s));
   }
-  CUfunction fn = gt_jit(tab, sizeof(T) == 8, r.fp_mode == PSB_FP_FMA, s, r.smem_optin);
+  CUfunction fn = gt_jit(tab, geo, sizeof(T) == 8, r.fp_mode == PSB_FP_FMA, s, r.smem_optin);
   GridView ov = og->view();
   if (fn) {
     void *args[] = {&maps, &tab, &ov, &d, &geo, &r.d_error};

@@ -464,4 +464,179 @@ __device__ __forceinline__ void gt_body(const GtMaps &maps, const GtTable &tab,
   for (int j = nzl; j < nplanes; j++) release(j);
 }
 
+// One staged row of the plane-by-plane form: the thread's vector and the
+// values beside it that the table reads (P2/P1 before it, N1/N2 after it).
+template <typename T, bool P2, bool P1, bool N1, bool N2>
+__device__ __forceinline__ void gt_row_ext(const T *p, int lane, GtRow<T> &r) {
+  constexpr int V = 16 / sizeof(T);
+  const Vec16<T> a = lds16(p);
+#pragma unroll
+  for (int j = 0; j < V; j++) r.e[2 + j] = a.v[j];
+  if constexpr (N1) r.e[V + 2] = __shfl_down_sync(0xffffffffu, a.v[0], 1);
+  if constexpr (N2) r.e[V + 3] = __shfl_down_sync(0xffffffffu, a.v[1], 1);
+  if constexpr (P2) r.e[0] = __shfl_up_sync(0xffffffffu, a.v[V - 2], 1);
+  if constexpr (P1) r.e[1] = __shfl_up_sync(0xffffffffu, a.v[V - 1], 1);
+  if constexpr (N1 || N2) {
+    if (lane == 31) {
+      if constexpr (N1) r.e[V + 2] = p[V];
+      if constexpr (N2) r.e[V + 3] = p[V + 1];
+    }
+  }
+  if constexpr (P1 || P2) {
+    if (lane == 0) {
+      if constexpr (P2) r.e[0] = p[-2];
+      if constexpr (P1) r.e[1] = p[-1];
+    }
+  }
+}
+
+// One term of the plane-by-plane form on a thread's rows of the plane (q[2 +
+// y]: row y of the block): its product added to the block's running sum
+// (FIRST: starts it), rounded as gt_term rounds it. SHARED: other terms have
+// the same coefficient, so scalar products are kept for them; products of a
+// coefficient of its own go in pairs where the values sit in aligned pairs
+// (27 distinct coefficients at 512^3: 360 us against 400; fused pairs were no
+// faster than scalar fused adds).
+template <typename T, int DY, int DXP2, bool ONE, bool FIRST, bool FMA, bool SHARED = true>
+__device__ __forceinline__ void gt_plane_term(const GtRow<T> *q, T c, GtBlk<T> &acc) {
+  if constexpr (sizeof(T) == 4 && !FMA && !ONE && !SHARED && DXP2 % 2 == 0) {
+    const float2 cc = make_float2(c, c);
+#pragma unroll
+    for (int r = 0; r < kGtVY; r++)
+#pragma unroll
+      for (int v = 0; v < 4; v += 2) {
+        const float2 x = make_float2(q[2 + r + DY].e[DXP2 + v], q[2 + r + DY].e[DXP2 + v + 1]);
+        const float2 y = __fmul2_rn(cc, x);
+        acc.v[r][v] = FIRST ? y.x : xadd(acc.v[r][v], y.x);
+        acc.v[r][v + 1] = FIRST ? y.y : xadd(acc.v[r][v + 1], y.y);
+      }
+    return;
+  }
+#pragma unroll
+  for (int r = 0; r < kGtVY; r++)
+#pragma unroll
+    for (int v = 0; v < 16 / (int)sizeof(T); v++) {
+      const T x = q[2 + r + DY].e[DXP2 + v];
+      if constexpr (FMA && !FIRST && !ONE) {
+        if constexpr (sizeof(T) == 4) acc.v[r][v] = __fmaf_rn(c, x, acc.v[r][v]);
+        else acc.v[r][v] = __fma_rn(c, x, acc.v[r][v]);
+      } else {
+        const T y = ONE ? x : xmul(c, x);
+        acc.v[r][v] = FIRST ? y : xadd(acc.v[r][v], y);
+      }
+    }
+}
+
+// Kernel body of packed tables whose terms come in the order of their planes
+// (z offsets never decrease): every input plane is taken once, as it arrives,
+// and adds its terms to the running sums of the Prog::kWindow output planes
+// that read it, which stay in registers. The window form (gt_body) reads each
+// plane from shared memory again for every output plane and every term row:
+// on the 27-point table 36 row loads, with their shuffles, per output plane
+// of a thread's four rows, against 6 here, and terms with equal coefficients
+// share their products.
+template <typename T, class Prog>
+__device__ __forceinline__ void gt_body_planes(const GtMaps &maps, const GtTable &tab,
+                                               const GridView &out, const Dom3 &d,
+                                               const GtGeom &geo, int *err) {
+  constexpr int V = 16 / sizeof(T), W = Prog::kWindow;
+  extern __shared__ __align__(128) unsigned char smem_raw[];
+  unsigned char *smem = smem_raw + ((128 - (smem_u32(smem_raw) & 127)) & 127);
+  uint64_t *full = reinterpret_cast<uint64_t *>(smem);
+  uint64_t *empty = full + 32;
+  unsigned char *ring = smem + 512;
+  const int S = geo.stages;
+  constexpr int TX = 32 * V, TY = (kGtConsumers / 32) * kGtVY;
+  int b = blockIdx.x;
+  const int tile_x = b % geo.tiles_x;
+  b /= geo.tiles_x;
+  const int tile_y = b % geo.tiles_y;
+  const int zc = b / geo.tiles_y;
+  const int x0 = geo.x_base + tile_x * TX;
+  const int y0 = d.lo[1] + tile_y * TY;
+  const int zb = d.lo[2] + zc * geo.zchunk;
+  const int nzl = min(zb + geo.zchunk, d.hi[2]) - zb;
+  const int nplanes = nzl + W - 1;
+  const int tid = threadIdx.x;
+  if (tid == 0) {
+    for (int i = 0; i < S; i++) {
+      mbar_init(&full[i], 1);
+      mbar_init(&empty[i], kGtConsumers / 32);
+    }
+    mbar_fence_init();
+  }
+  __syncthreads();
+
+  if (tid >= kGtConsumers) {
+    if (tid != kGtConsumers) return;
+    for (int g = 0; g < geo.ngrids; g++) tma_prefetch_desc(&maps.m[g]);
+    const uint32_t bytes = (uint32_t)(geo.ngrids * geo.bx * geo.by * sizeof(T));
+    RingPos p{0, 0};
+    for (int j = 0; j < nplanes; j++) {
+      if (p.round > 0 && !mbar_wait_bounded(&empty[p.slot], (p.round - 1) & 1)) {
+        atomicExch(err, 1);
+        ring_drain(Ring{full, empty, ring, S, geo.stage_bytes}, p);
+        return;
+      }
+      mbar_arrive_expect_tx(&full[p.slot], bytes);
+      const int z = zb + geo.zmin + j;
+      unsigned char *dst = ring + (size_t)p.slot * geo.stage_bytes;
+      for (int g = 0; g < geo.ngrids; g++)
+        tma_load_3d(dst + (size_t)g * geo.plane_elems * sizeof(T), &maps.m[g], &full[p.slot],
+                    x0 - V + geo.ax0[g], y0 - kGtR + geo.ay0[g], z + geo.az0[g]);
+      ring_next(p, S);
+    }
+    return;
+  }
+
+  const int lane = tid & 31, ty = tid >> 5;
+  const int xg0 = x0 + lane * V, yg0 = y0 + ty * kGtVY;
+  const int thr_off = (ty * kGtVY + kGtR) * geo.bx + V + lane * V;
+  const bool xvec = geo.vec_store && xg0 >= d.lo[0] && xg0 + V <= d.hi[0];
+  bool row_in[kGtVY];
+#pragma unroll
+  for (int r = 0; r < kGtVY; r++) row_in[r] = yg0 + r >= d.lo[1] && yg0 + r < d.hi[1];
+  T *dst0 = (T *)out.origin + (int64_t)xg0 + (int64_t)yg0 * out.sy + (int64_t)zb * out.sz;
+
+  // acc[(W - k) % W]: the running sums of output plane j - k at input plane
+  // j, which takes its terms of window plane k. They shift by moves after each
+  // plane: a loop unrolled over the W roles outgrows the instruction cache
+  // (27 coefficients at 512^3: 249 us against 239).
+  GtBlk<T> acc[W];
+  RingPos pos{0, 0};
+#pragma unroll 1
+  for (int j = 0; j < nplanes; j++) {
+    if (!__all_sync(0xffffffffu, mbar_wait_bounded(&full[pos.slot], pos.round & 1))) {
+      if (lane == 0) atomicExch(err, 1);
+      return;
+    }
+    const T *stage = reinterpret_cast<const T *>(ring + (size_t)pos.slot * geo.stage_bytes);
+    Prog::template plane<T>(tab, stage + thr_off, geo.bx, geo.plane_elems, lane, acc);
+    __syncwarp();
+    if (lane == 0) mbar_arrive(&empty[pos.slot]);
+    ring_next(pos, S);
+    if (j >= W - 1) {
+      const GtBlk<T> &o = acc[1];
+#pragma unroll
+      for (int r = 0; r < kGtVY; r++) {
+        if (!row_in[r]) continue;
+        T *dst = dst0 + r * out.sy;
+        if (xvec) {
+          Vec16<T> w;
+#pragma unroll
+          for (int v = 0; v < V; v++) w.v[v] = o.v[r][v];
+          stg16(dst, w);
+        } else {
+#pragma unroll
+          for (int v = 0; v < V; v++)
+            if (xg0 + v >= d.lo[0] && xg0 + v < d.hi[0]) dst[v] = o.v[r][v];
+        }
+      }
+      dst0 += out.sz;
+    }
+#pragma unroll
+    for (int k = 1; k < W; k++) acc[k] = acc[(k + 1) % W];
+  }
+}
+
 }  // namespace psb
