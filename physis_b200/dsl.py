@@ -634,50 +634,49 @@ __device__ __forceinline__ int __psb_dim(const __psb_grid<T> &g, int d) {
 // a grid read from the staged window at an offset from the point in row r,
 // column v of the thread's block, and the grid emitted into, whose value
 // goes to that point's result.
-// A read grid of the staged form: the rows the function reads around the
-// current row of the thread's block, in registers (L::id maps a row's grid,
-// dy and dz to its index), and the point's column v in that row. Unchecked
-// (C false): the library runs it only when every read the function can make
-// over the map's domain lies inside its grid. Checked (C true): a read that
-// leaves the point on an axis is tested against the grid there and, outside,
-// reads 0 and marks the thread's flag (*bad), which the program turns into
-// PSB_ERR_BOUNDS once per thread like the function's own form reports it.
-// The library runs it only with the domain inside the grid, so a read at
-// the point's own coordinate on an axis needs no test (the offsets are
-// constants after inlining, so each read keeps the tests of its own axes).
-// The test is a select, not a branch, so the points of a thread's block
-// still schedule together.
-template <typename T, class L, bool C>
+// A read grid of the staged form: the rows of the thread's block that the
+// function reads, in registers (L::id maps a grid, the point's row r in the
+// block, dy and dz to a row), and the point's row r and column v. CX, CY, CZ:
+// a read that leaves the point on that axis is tested against the grid there
+// and, outside, reads 0 and marks the thread's flag (*bad), which the program
+// turns into PSB_ERR_BOUNDS once per thread like the function's own form
+// reports it; unset where the library or the program knows that no read of
+// these points can leave the grid on that axis. Checked forms run only with
+// the domain inside the grid, so a read at the point's own coordinate on an
+// axis needs no test (the offsets are constants after inlining). The test is
+// a select, not a branch, so the points of a thread's block still schedule
+// together.
+template <typename T, class L, bool CX, bool CY, bool CZ>
 struct __psb_rgrid {
   const psb::GtRow<T> *rows;
-  int slot, v, x, y, z;
+  int slot, r, v, x, y, z;
   int n0, n1, n2;
   int *bad;
 };
 
-template <typename T, class L, bool C>
-__device__ __forceinline__ T __psb_get(const __psb_rgrid<T, L, C> &g, int i, int j = 0,
+template <typename T, class L, bool CX, bool CY, bool CZ>
+__device__ __forceinline__ T __psb_get(const __psb_rgrid<T, L, CX, CY, CZ> &g, int i, int j = 0,
                                        int k = 0) {
   const int dx = i - g.x, dy = j - g.y, dz = k - g.z;
-  const T val = g.rows[L::id(g.slot, dy, dz)].e[2 + dx + g.v];
-  if (!C) return val;
-  const bool out = ((dx != 0) & ((unsigned)i >= (unsigned)g.n0)) |
-                   ((dy != 0) & ((unsigned)j >= (unsigned)g.n1)) |
-                   ((dz != 0) & ((unsigned)k >= (unsigned)g.n2));
+  const T val = g.rows[L::id(g.slot, g.r, dy, dz)].e[2 + dx + g.v];
+  if (!CX && !CY && !CZ) return val;
+  const bool out = (CX & (dx != 0) & ((unsigned)i >= (unsigned)g.n0)) |
+                   (CY & (dy != 0) & ((unsigned)j >= (unsigned)g.n1)) |
+                   (CZ & (dz != 0) & ((unsigned)k >= (unsigned)g.n2));
   *g.bad |= (int)out;
   return out ? T(0) : val;
 }
 
 // A periodic read: the window holds the wrapped values (the library
 // refreshes the pitched grid's halo first), so it needs no check.
-template <typename T, class L, bool C>
-__device__ __forceinline__ T __psb_getp(const __psb_rgrid<T, L, C> &g, int i, int j = 0,
+template <typename T, class L, bool CX, bool CY, bool CZ>
+__device__ __forceinline__ T __psb_getp(const __psb_rgrid<T, L, CX, CY, CZ> &g, int i, int j = 0,
                                         int k = 0) {
-  return g.rows[L::id(g.slot, j - g.y, k - g.z)].e[2 + (i - g.x) + g.v];
+  return g.rows[L::id(g.slot, g.r, j - g.y, k - g.z)].e[2 + (i - g.x) + g.v];
 }
 
-template <typename T, class L, bool C>
-__device__ __forceinline__ int __psb_dim(const __psb_rgrid<T, L, C> &g, int d) {
+template <typename T, class L, bool CX, bool CY, bool CZ>
+__device__ __forceinline__ int __psb_dim(const __psb_rgrid<T, L, CX, CY, CZ> &g, int d) {
   return d == 0 ? g.n0 : (d == 1 ? g.n1 : g.n2);
 }
 
@@ -911,44 +910,89 @@ def _staged_function(info, params, body):
         ", ".join(tpl), info.name, ", ".join(args), body)
 
 
+# Rows of a thread's block in the staged form (kGtVY of k_generic_tma.cuh),
+# and the reads up to which a checked function gets a copy per kind of block.
+_BLOCK_ROWS = 4
+_COPIES_MAX_READS = 14
+
+
 def _staged_entry(info):
     """The point-wise program, kernels and launchers of the staged form,
     unchecked and checked (psb_dsl_staged_<name>, psb_dsl_staged_checked_<name>).
 
-    For each row of the thread's block the rows the function reads -- one
-    per (grid, dy, dz) -- are loaded into registers as the generic packed
-    form does (a 16-byte load per thread, x neighbours from the adjacent
-    lanes); every read of the function then resolves, at compile time, to a
-    register of one of those rows. The checked form tests the reads that
-    leave the point against their grids first (rows outside a grid hold
-    whatever the window holds there and are never returned)."""
+    The rows the function reads around the thread's block are loaded into
+    registers as the generic packed form does (a 16-byte load per thread, x
+    neighbours from the adjacent lanes); every read of the function then
+    resolves, at compile time, to a register of one of those rows. The checked
+    form tests the reads that leave the point against their grids first (rows
+    outside a grid hold whatever the window holds there and are never
+    returned).
+
+    Functions of few reads load every row of the block once, and their checked
+    form is compiled for each kind of block: in y and z at least two points
+    inside every grid and inside the domain, or not, and in x the same, a
+    vector inside the domain, or neither. The compiler is told what holds and
+    drops the function's own face tests with the read and domain tests, which
+    were 80 of 93 instructions per point on the diffusion function. Functions of
+    many reads keep one copy and load the rows of one block row at a time:
+    copies of a large body outgrow the instruction cache, and all rows at once
+    the registers (27-point box at 512^3: 883 us a step against 668)."""
     n = info.name
     t = _CTYPE[info.gparams[0].ctype]
     rows = list(info.staged_rows.items())
-    ids = " : ".join("(slot == %d && dy == %d && dz == %d) ? %d" % (sl, dy, dz, k)
-                     for k, ((sl, dy, dz), _) in enumerate(rows)) + " : 0"
+    few = sum(hi - lo + 1 for lo, hi in info.staged_rows.values()) <= _COPIES_MAX_READS
+    planes, flags = [], {}
+    for (sl, dy, dz), (dxlo, dxhi) in rows:
+        if (sl, dz) not in planes:
+            planes.append((sl, dz))
+        for r in range(_BLOCK_ROWS):
+            f = flags.setdefault((sl, dz, r + dy), [False] * 4)
+            for i, need in enumerate((dxlo <= -2, dxlo <= -1, dxhi >= 1, dxhi >= 2)):
+                f[i] = f[i] or need
+    span = _BLOCK_ROWS + 4
+    stage = ("const T *p = reinterpret_cast<const T *>(at.ring + (size_t)sl * at.sbytes) + "
+             "tab.slot_grid[%d] * at.plane_elems + at.thr_off;")
+    wrap = "int sl = at.slot0 + %d - at.zmin; if (sl >= at.S) sl -= at.S; "
     loads = []
-    for k, ((sl, dy, dz), (dxlo, dxhi)) in enumerate(rows):
-        loads.append(
-            "{ int sl = at.slot0 + %d - at.zmin; if (sl >= at.S) sl -= at.S;\n"
-            "          psb::gt_row_load(reinterpret_cast<const T *>(at.ring + (size_t)sl * at.sbytes) + "
-            "tab.slot_grid[%d] * at.plane_elems + at.thr_off + (r + %d) * at.bx, lane, %s, %s, "
-            "rows[%d]); }" % (dz, sl, dy, "true" if dxhi > 0 else "false",
-                              "true" if dxlo < 0 else "false", k))
-    handles, args = [], []
+    if few:
+        ids = " : ".join("(slot == %d && dz == %d) ? %d + r + dy" % (sl, dz, k * span + 2)
+                         for k, (sl, dz) in enumerate(planes)) + " : 0"
+        for k, (sl, dz) in enumerate(planes):
+            loads.append("{ " + wrap % dz + stage % sl)
+            for (s2, z2, y), f in flags.items():
+                if (s2, z2) == (sl, dz):
+                    loads.append("  psb::gt_row_ext<T, %s>(p + (%d) * at.bx, lane, rows[%d]);" % (
+                        ", ".join("true" if b else "false" for b in f), y, k * span + 2 + y))
+            loads.append("}")
+    else:
+        ids = " : ".join("(slot == %d && dy == %d && dz == %d) ? %d" % (sl, dy, dz, k)
+                         for k, ((sl, dy, dz), _) in enumerate(rows)) + " : 0"
+        for k, ((sl, dy, dz), (dxlo, dxhi)) in enumerate(rows):
+            loads.append("{ " + wrap % dz + stage % sl + " psb::gt_row_load(p + (r + %d) * at.bx, "
+                         "lane, %s, %s, rows[%d]); }" % (dy, "true" if dxhi > 0 else "false",
+                                                         "true" if dxlo < 0 else "false", k))
+    handles, args, known = [], [], {"x": [], "y": [], "z": []}
+    inside = {"x": ["at.x >= 2"], "y": ["at.y >= 2"], "z": ["at.z >= 2"]}
+    ends = {"x": "at.x + V + 2", "y": "at.y + psb::kGtVY + 2", "z": "at.z + 3"}
     for slot in range(len(info.gparams)):
         dims = ", ".join("tab.slot_dims[%d][%d]" % (slot, k) for k in range(3))
         if slot == info.emit_slot:
             handles.append("const __psb_ogrid<T> g%d{&acc.v[r][v], %s};" % (slot, dims))
         else:
-            handles.append("const __psb_rgrid<T, __psb_rows_%s, C> g%d{rows, %d, v, x, y, at.z, "
-                           "%s, &bad};" % (n, slot, slot, dims))
+            handles.append("const __psb_rgrid<T, __psb_rows_%s, C && X != 2, C && !YZ, C && !YZ> "
+                           "g%d{rows, %d, r, v, x, y, z, %s, &bad};" % (n, slot, slot, dims))
+        for k, ax in enumerate("xyz"):
+            d = "tab.slot_dims[%d][%d]" % (slot, k)
+            inside[ax].append("%s <= %s" % (ends[ax], d))
+            known[ax] += ["__builtin_assume(%s < %s - %d);" % (ax, d, m) for m in (2, 1)]
         args.append("g%d" % slot)
+    for ax in "xyz":
+        known[ax] += ["__builtin_assume(%s >= 2);" % ax, "__builtin_assume(%s > 0);" % ax]
     for k, (_, st) in enumerate(info.scalars):
         args.append("(%s)tab.coef[%d]" % (_CTYPE[st], k))
     return """
 struct __psb_rows_{n} {{
-  static __device__ __forceinline__ constexpr int id(int slot, int dy, int dz) {{
+  static __device__ __forceinline__ constexpr int id(int slot, int r, int dy, int dz) {{
     return {ids};
   }}
 }};
@@ -960,36 +1004,70 @@ struct __psb_prog_{n} {{
   template <typename T>
   static __device__ __forceinline__ void eval(const psb::GtTable &, const unsigned char *, int,
                                               int, int, int, int, int, psb::GtBlk<T> &) {{}}
+  // The points of the block. X: 2 the block lies inside the domain and at
+  // least two points inside every grid in x, 1 inside the domain in x, 0
+  // neither is known. YZ: as X = 2 in y and z.
+  template <int X, bool YZ, typename T>
+  static __device__ __forceinline__ void points(const psb::GtTable &tab, const psb::GtAt &at,
+                                                psb::GtRow<T> (&rows)[{nrows}], int &bad,
+                                                psb::GtBlk<T> &acc) {{
+    const int z = at.z, lane = threadIdx.x & 31;
+    (void)lane;
+    if constexpr (YZ) {{
+      {known_z}
+    }}
+#pragma unroll
+    for (int r = 0; r < psb::kGtVY; r++) {{
+      {loads_r}
+      const int y = at.y + r;
+      if constexpr (YZ) {{
+        {known_y}
+      }} else if (y < at.lo1 || y >= at.hi1) {{
+        continue;
+      }}
+#pragma unroll
+      for (int v = 0; v < 16 / (int)sizeof(T); v++) {{
+        const int x = at.x + v;
+        if constexpr (X == 2) {{
+          {known_x}
+        }} else if (X == 0 && (x < at.lo0 || x >= at.hi0)) {{
+          continue;
+        }}
+        {handles}
+        {n}__staged(x, y, z, {args});
+      }}
+    }}
+  }}
   template <typename T>
   static __device__ __forceinline__ void eval_points(const psb::GtTable &tab,
                                                      const psb::GtAt &at, psb::GtBlk<T> &acc) {{
     const int lane = threadIdx.x & 31;
+    (void)lane;
     int bad = 0;  // a checked read of this thread's block left its grid
-#pragma unroll
-    for (int r = 0; r < psb::kGtVY; r++) {{
-      psb::GtRow<T> rows[{nrows}];  // every lane loads: the rows share values by shuffles
-      {loads}
-      const int y = at.y + r;
-      if (y < at.lo1 || y >= at.hi1) continue;
-#pragma unroll
-      for (int v = 0; v < 16 / (int)sizeof(T); v++) {{
-        const int x = at.x + v;
-        if (x < at.lo0 || x >= at.hi0) continue;
-        {handles}
-        {n}__staged(x, y, at.z, {args});
-      }}
+    psb::GtRow<T> rows[{nrows}];
+    {loads}
+    if constexpr (C && {copies}) {{
+      constexpr int V = 16 / (int)sizeof(T);
+      const bool yz = at.y >= at.lo1 && at.y + psb::kGtVY <= at.hi1 && {in_yz};
+      const bool dx = at.x >= at.lo0 && at.x + V <= at.hi0, ix = dx && {in_x};
+      if (yz && __all_sync(0xffffffffu, ix)) points<2, true>(tab, at, rows, bad, acc);
+      else if (yz && dx) points<1, true>(tab, at, rows, bad, acc);
+      else if (at.x < at.hi0 && at.x + V > at.lo0)  // not wholly outside
+        points<0, false>(tab, at, rows, bad, acc);
+    }} else {{
+      points<0, false>(tab, at, rows, bad, acc);
     }}
     if (C && bad) atomicExch(tab.read_err, (int)PSB_ERR_BOUNDS);
   }}
 }};
 
-extern "C" __global__ void __launch_bounds__(psb::kGtThreads, 2) __psb_staged_kernel_{n}(
+extern "C" __global__ void __launch_bounds__(psb::kGtThreads, {minb}) __psb_staged_kernel_{n}(
     const __grid_constant__ psb::GtMaps maps, const __grid_constant__ psb::GtTable tab,
     psb::GridView out, psb::Dom3 d, const __grid_constant__ psb::GtGeom geo, int *err) {{
   psb::gt_body<{t}, __psb_prog_{n}<false>>(maps, tab, out, d, geo, err);
 }}
 
-extern "C" __global__ void __launch_bounds__(psb::kGtThreads, 2) __psb_staged_checked_kernel_{n}(
+extern "C" __global__ void __launch_bounds__(psb::kGtThreads, {minb}) __psb_staged_checked_kernel_{n}(
     const __grid_constant__ psb::GtMaps maps, const __grid_constant__ psb::GtTable tab,
     psb::GridView out, psb::Dom3 d, const __grid_constant__ psb::GtGeom geo, int *err) {{
   psb::gt_body<{t}, __psb_prog_{n}<true>>(maps, tab, out, d, geo, err);
@@ -1032,8 +1110,13 @@ extern "C" psb_status psb_dsl_staged_checked_{n}(const void *maps, const void *t
   return __psb_staged_launch_{n}(__psb_staged_checked_kernel_{n}, &configured, maps, table, out,
                                  dom, geo, err, blocks, smem, stream);
 }}
-""".format(n=n, t=t, ids=ids, nrows=len(rows), loads="\n      ".join(loads),
-           handles="\n        ".join(handles), args=", ".join(args))
+""".format(n=n, t=t, ids=ids, nrows=len(planes) * span if few else len(rows),
+           loads="\n    ".join(loads if few else []),
+           loads_r="\n      ".join([] if few else loads), copies="true" if few else "false",
+           minb=3 if few else 2, handles="\n        ".join(handles), args=", ".join(args),
+           in_x=" && ".join(inside["x"]), in_yz=" && ".join(inside["y"] + inside["z"]),
+           known_x="\n          ".join(known["x"]), known_y="\n        ".join(known["y"]),
+           known_z="\n      ".join(known["z"]))
 
 
 def _read_ranges(info):
