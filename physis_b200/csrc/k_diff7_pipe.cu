@@ -110,15 +110,31 @@ psb_status diff7_pipe_launch(MapImpl &m, GridImpl *in, GridImpl *out, const Pipe
 }
 
 // --------------------------------------------------------------------------
-// Choice of the passes' shape. A walk's turn takes what its SM's warps issue
-// (a row-stage is one row of one stage of one warp) or the latency of its
-// stages, which run one after the other, whichever is longer, plus part of
-// the other; a pass takes its full waves of CTAs and the last one. The
-// constants (cycles) are fitted to some 10,000 timed shapes (64^3 to 512^3 and
-// ragged extents, float and double, exact and FMA): the shape chosen takes 3
-// to 4% more than the fastest timed one on average. Small tiles spread over
-// more SMs but recompute more halo.
+// Choice of the passes' shape. A turn of a walk takes what its SM's warps
+// issue (row-stages: one row of one stage of one warp) or the latency of its
+// stages, whichever is longer, and `both` of the other; a walk its planes and
+// `extra` turns, and in periodic passes the copies of the images after it; a
+// pass its full waves of CTAs, the last one and its launch. The constants
+// (cycles) are fitted to 10,000 timed shapes (33x40x300 to 512^3 with ragged
+// extents): estimates are off by 6 to 12% on average, and the shape chosen
+// takes 1 to 4% more than the fastest one timed. Small tiles spread over more
+// SMs but recompute more halo.
 // --------------------------------------------------------------------------
+struct PipeFit {
+  double row_stage, latency, both, extra, launch, images;
+};
+
+static const PipeFit &pipe_fit(int ns, bool dbl, bool per, bool fast) {
+  // [double][FMA]
+  static const PipeFit two[2][2] = {{{53.6, 1262, 0.83, 3.1, 8900, 0}, {44.5, 1228, 0.83, 3.1, 7200, 0}},
+                                    {{47.5, 916, 0.69, 4.7, 8100, 0}, {43.0, 862, 0.71, 3.9, 7000, 0}}};
+  static const PipeFit four[2][2] = {{{32.9, 1280, 0.92, 6.7, 9100, 0}, {31.1, 1015, 0.95, 6.2, 9100, 0}},
+                                     {{39.7, 846, 0.81, 9.0, 10800, 0}, {38.5, 783, 0.77, 8.2, 9200, 0}}};
+  static const PipeFit wrap[2][2] = {{{75.3, 1595, 0.64, 2.2, 9300, 42}, {49.3, 1693, 0.82, 2.0, 8700, 108}},
+                                     {{45.8, 1117, 0.76, 4.1, 9200, 85}, {49.8, 1210, 0.17, 5.5, 7500, 242}}};
+  return per ? wrap[dbl][fast] : ns == 4 ? four[dbl][fast] : two[dbl][fast];
+}
+
 static double pipe_cost(const PipeConfig &c, bool dbl, bool per, bool fast, const int *n) {
   const int V = dbl ? 2 : 4, w = V << c.xl_shift;
   const int rows = (c.threads >> c.xl_shift) * c.r;
@@ -131,19 +147,15 @@ static double pipe_cost(const PipeConfig &c, bool dbl, bool per, bool fast, cons
                       (size_t)(c.ns - 1) * 64 * c.threads;
   const int occ = (int)std::min<size_t>(65536 / (168 * c.threads), (228 << 10) / smem);
   if (occ < 1) return -1;
-  const int64_t per_wave = (int64_t)rt().sm_count * occ;
-  const double row_stage = per ? (dbl ? 55 : 60) : dbl ? (fast ? 44 : 50) : (fast ? 60 : 70);
-  const double latency = 150 + (per ? 500.0 : dbl && c.ns == 4 ? 220.0 : 300.0) * c.ns;
-  const double both = per && !dbl ? 0.7 : 0.4;
-  const double images = per ? 160.0 * c.zchunk * rows / c.threads : 0;  // copied after the walk
+  const PipeFit &f = pipe_fit(c.ns, dbl, per, fast);
   auto walk = [&](int64_t resident) {  // CTAs on the busiest SM
-    const double issue = row_stage * c.ns * c.r * std::max(1.0, resident * c.threads / 128.0);
-    return (c.zchunk + 1.5 * c.ns + 3) *
-               (std::max(issue, latency) + both * std::min(issue, latency)) +
-           images * resident;
+    const double issue = f.row_stage * c.ns * c.r * std::max(1.0, resident * c.threads / 128.0);
+    return (c.zchunk + f.extra) *
+               (std::max(issue, f.latency) + f.both * std::min(issue, f.latency)) +
+           f.images * c.zchunk * rows / c.threads * resident;
   };
-  const int64_t rest = blocks % per_wave;
-  return 5500 + (double)(blocks / per_wave) * walk(occ) +
+  const int64_t per_wave = (int64_t)rt().sm_count * occ, rest = blocks % per_wave;
+  return f.launch + (double)(blocks / per_wave) * walk(occ) +
          (rest ? walk((rest + rt().sm_count - 1) / rt().sm_count) : 0.0);
 }
 

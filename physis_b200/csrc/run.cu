@@ -374,10 +374,12 @@ static bool pipe_plan(MapImpl **ms, int iter, PipePlan *plan) {
     plan->singles = steps - 2 * plan->twos;
     return plan->twos > 0;
   }
-  // A single step: its launch, and its bytes at about the L2 rate while both
-  // grids fit, the HBM rate beyond (cycles).
+  // A single step (cycles): its launch, and the points of its 32 x 16 tiles
+  // at the rate measured while both grids stay in L2 and beyond (float 230
+  // and 360 points a cycle, double 160 and 190).
   const double bytes = 2.0 * A->pub.elm_size * A->pub.num_elms;
-  const double t1 = 6000 + bytes / (bytes < 100e6 ? 2000.0 : 3000.0);
+  const double rate = bytes < 100e6 ? (dbl ? 160 : 230) : (dbl ? 190 : 360);
+  const double t1 = 7500 + ((n[0] + 31) / 32 * 32.0) * ((n[1] + 15) / 16 * 16.0) * n[2] / rate;
   double best = t1 * steps;
   for (int c = 1; c <= 3 && c <= steps; c += 2)
     for (int b = 0; 2 * b <= steps - c; b++) {
