@@ -39,14 +39,15 @@ static psb_status pipe_launch(MapImpl &m, GridImpl *in, GridImpl *out, const Pip
   g.rows = cfg.threads / xl * R;
   g.bx = std::min(w, 256);
   g.nbox = w / g.bx;
-  if (g.rows > 256 || g.rows <= 2 * NS || w <= 2 * NS + V) return PSB_ERR_INVALID;
-  const int hx = (NS + V - 1) / V * V;  // tile starts stay on 16 bytes
+  if (g.rows > 256 || g.rows <= 2 * NS || w <= 2 * pipe_hx(NS, V) + V) return PSB_ERR_INVALID;
+  const int hx = (NS + V - 1) / V * V;  // periodic tiles start this far before x = 0
   g.ex0 = PERIODIC ? -hx : 0;
   g.ey0 = PERIODIC ? -NS : 0;
-  g.sx = w - 2 * NS;
+  constexpr int HX = pipe_hx(NS, V);
+  g.sx = w - 2 * HX;
   g.sy = g.rows - 2 * NS;
   if (g.sx % V) return PSB_ERR_INVALID;
-  g.tiles_x = pipe_tiles(n[0], w, NS, PERIODIC, hx);
+  g.tiles_x = pipe_tiles(n[0], w, HX, PERIODIC, hx);
   g.tiles_y = pipe_tiles(n[1], g.rows, NS, PERIODIC, NS);
   g.zchunk = std::max(1, cfg.zchunk);
   const int nzc = (n[2] + g.zchunk - 1) / g.zchunk;
@@ -102,9 +103,12 @@ psb_status diff7_pipe_launch(MapImpl &m, GridImpl *in, GridImpl *out, const Pipe
     if (dbl) return per ? PSB_PIPE(double, 2, 4, 192, 2, true) : PSB_PIPE(double, 2, 4, 192, 2, false);
     return per ? PSB_PIPE(float, 2, 4, 192, 2, true) : PSB_PIPE(float, 2, 4, 192, 2, false);
   }
-  // Four steps need four halo cells; a periodic grid keeps two.
+  // More than two steps need more halo than the two cells a periodic grid
+  // keeps.
   if (cfg.ns == 4 && cfg.r == 2 && !per)
     return dbl ? PSB_PIPE(double, 4, 2, 384, 1, false) : PSB_PIPE(float, 4, 2, 384, 1, false);
+  if (cfg.ns == 3 && cfg.r == 2 && !per)
+    return dbl ? PSB_PIPE(double, 3, 2, 384, 1, false) : PSB_PIPE(float, 3, 2, 384, 1, false);
 #undef PSB_PIPE
   return PSB_ERR_INVALID;
 }
@@ -132,15 +136,14 @@ static const PipeFit &pipe_fit(int ns, bool dbl, bool per, bool fast) {
                                      {{39.7, 846, 0.81, 9.0, 10800, 0}, {38.5, 783, 0.77, 8.2, 9200, 0}}};
   static const PipeFit wrap[2][2] = {{{75.3, 1595, 0.64, 2.2, 9300, 42}, {49.3, 1693, 0.82, 2.0, 8700, 108}},
                                      {{45.8, 1117, 0.76, 4.1, 9200, 85}, {49.8, 1210, 0.17, 5.5, 7500, 242}}};
-  return per ? wrap[dbl][fast] : ns == 4 ? four[dbl][fast] : two[dbl][fast];
+  return per ? wrap[dbl][fast] : ns > 2 ? four[dbl][fast] : two[dbl][fast];
 }
 
 static double pipe_cost(const PipeConfig &c, bool dbl, bool per, bool fast, const int *n) {
   const int V = dbl ? 2 : 4, w = V << c.xl_shift;
   const int rows = (c.threads >> c.xl_shift) * c.r;
-  if (rows <= 2 * c.ns || rows > 256 || w <= 2 * c.ns + V) return -1;
-  const int hx = (c.ns + V - 1) / V * V;
-  const int64_t tiles = (int64_t)pipe_tiles(n[0], w, c.ns, per, hx) *
+  if (rows <= 2 * c.ns || rows > 256 || w <= 2 * pipe_hx(c.ns, V) + V) return -1;
+  const int64_t tiles = (int64_t)pipe_tiles(n[0], w, pipe_hx(c.ns, V), per, (c.ns + V - 1) / V * V) *
                         pipe_tiles(n[1], rows, c.ns, per, c.ns);
   const int64_t blocks = tiles * ((n[2] + c.zchunk - 1) / c.zchunk);
   const size_t smem = 1280 + (size_t)c.stages * w * rows * (dbl ? 8 : 4) +
@@ -177,10 +180,10 @@ PipeConfig diff7_pipe_choose(int ns, bool dbl, bool per, bool fast, const int *n
     PipeConfig best{};
     double best_cost = -1;
     for (int shift = 3; shift <= 5; shift++)
-      for (int threads = 64; threads <= (ns == 4 ? 384 : 192); threads += 32) {
+      for (int threads = 64; threads <= (ns > 2 ? 384 : 192); threads += 32) {
         if (threads % (1 << shift)) continue;
         for (int nc = 1; nc <= std::max(1, n[2] / 4) && nc <= 64; nc++) {
-          const PipeConfig c{ns, ns == 4 ? 2 : 4, threads, shift, (n[2] + nc - 1) / nc, 4};
+          const PipeConfig c{ns, ns > 2 ? 2 : 4, threads, shift, (n[2] + nc - 1) / nc, 4};
           const double t = pipe_cost(c, dbl, per, fast, n);
           if (t > 0 && (best_cost < 0 || t < best_cost)) {
             best = c;

@@ -46,6 +46,13 @@ struct PipeGeom {
   int stages, plane_bytes;
 };
 
+// Points at each x end of an extended tile that it does not store: the NS
+// that become invalid, rounded up where tile starts, NS apart from a multiple
+// of the vector, would leave 16 bytes.
+__host__ __device__ constexpr int pipe_hx(int ns, int v) {
+  return 2 * ns % v == 0 ? ns : (ns + v - 1) / v * v;
+}
+
 template <int I>
 struct PipeIdx {
   static constexpr int value = I;
@@ -56,6 +63,7 @@ __device__ __forceinline__ void diff7_pipe(const CUtensorMap *tin, const GridVie
                                            int ny, int nz, const C7<T> k7, const PipeGeom geo,
                                            int *err, unsigned char *smem) {
   constexpr int V = Vec16<T>::N;
+  constexpr int HX = pipe_hx(NS, V);
   const int S = geo.stages;
   uint64_t *full = reinterpret_cast<uint64_t *>(smem);
   unsigned char *ring = smem + 128;
@@ -83,13 +91,13 @@ __device__ __forceinline__ void diff7_pipe(const CUtensorMap *tin, const GridVie
   // The points this tile stores.
   int xlo, xhi, ylo, yhi;
   if (PERIODIC) {
-    xlo = max(0, xe + NS);
-    xhi = min(nx, xe + W - NS);
+    xlo = max(0, xe + HX);
+    xhi = min(nx, xe + W - HX);
     ylo = max(0, yt + NS);
     yhi = min(ny, yt + geo.rows - NS);
   } else {
-    xlo = xe == 0 ? 0 : xe + NS;
-    xhi = xe + W >= nx ? nx : xe + W - NS;
+    xlo = xe == 0 ? 0 : xe + HX;
+    xhi = xe + W >= nx ? nx : xe + W - HX;
     ylo = yt == 0 ? 0 : yt + NS;
     yhi = yt + geo.rows >= ny ? ny : yt + geo.rows - NS;
   }

@@ -337,14 +337,15 @@ static bool pipe_pair(MapImpl **ms, int n) {
   return true;
 }
 
-// How a run of `iter` pairs is cut: passes of four and two steps and single
-// steps, alternating A -> B and B -> A. Both grids have to end as after
+// How a run of `iter` pairs is cut: passes of four, three and two steps and
+// single steps, alternating A -> B and B -> A. Both grids have to end as after
 // single steps (A the last step, B the one before it), so the last step is a
-// single one from B, and the passes before it, 2 iter - 1 steps, are an odd
-// number of launches (three singles where one does not come out odd).
+// single one from B, and the 2 iter - 1 steps before it are an odd number of
+// launches.
 struct PipePlan {
-  PipeConfig four, two;
-  int fours = 0, twos = 0, singles = 0;
+  PipeConfig pass[5];  // by steps
+  int count[5] = {};   // [1]: single steps, besides the last one
+  int passes() const { return count[2] + count[3] + count[4]; }
 };
 
 // False: the run keeps single steps. A tune entry of a clamped float shape
@@ -365,14 +366,17 @@ static bool pipe_plan(MapImpl **ms, int iter, PipePlan *plan) {
     free_choice = cfg.tile_y == 16;
   }
   const int steps = 2 * iter - 1;  // before the last one
-  double t4 = -1, t2 = -1;
-  if (free_choice && !per) plan->four = diff7_pipe_choose(4, dbl, per, fast, n, &t4);
-  plan->two = diff7_pipe_choose(2, dbl, per, fast, n, &t2);
+  double t4 = -1, t3 = -1, t2 = -1;
+  if (free_choice && !per) {
+    plan->pass[4] = diff7_pipe_choose(4, dbl, per, fast, n, &t4);
+    plan->pass[3] = diff7_pipe_choose(3, dbl, per, fast, n, &t3);
+  }
+  plan->pass[2] = diff7_pipe_choose(2, dbl, per, fast, n, &t2);
   if (t2 < 0) return false;
   if (!free_choice) {
-    plan->twos = (iter - 1) & ~1;
-    plan->singles = steps - 2 * plan->twos;
-    return plan->twos > 0;
+    plan->count[2] = (iter - 1) & ~1;
+    plan->count[1] = steps - 2 * plan->count[2];
+    return plan->count[2] > 0;
   }
   // A single step (cycles): its launch, and the points of its 32 x 16 tiles
   // at the rate measured while both grids stay in L2 and beyond (float 230
@@ -380,22 +384,28 @@ static bool pipe_plan(MapImpl **ms, int iter, PipePlan *plan) {
   const double bytes = 2.0 * A->pub.elm_size * A->pub.num_elms;
   const double rate = bytes < 100e6 ? (dbl ? 160 : 230) : (dbl ? 190 : 360);
   const double t1 = 7500 + ((n[0] + 31) / 32 * 32.0) * ((n[1] + 15) / 16 * 16.0) * n[2] / rate;
+  // Two four-step passes beat any other eight steps in an even number of
+  // launches, so few of the others are needed.
   double best = t1 * steps;
-  for (int c = 1; c <= 3 && c <= steps; c += 2)
-    for (int b = 0; 2 * b <= steps - c; b++) {
-      const int left = steps - c - 2 * b;
-      if (left % 4 || (left && t4 < 0)) continue;
-      const int a = left / 4;
-      if ((a + b + c) % 2 == 0) continue;
-      const double t = a * t4 + b * t2 + c * t1;
-      if (t < best) {
-        best = t;
-        plan->fours = a;
-        plan->twos = b;
-        plan->singles = c;
+  for (int c = 0; c <= 3 && c <= steps; c++)
+    for (int d = 0; d <= 2 && c + 3 * d <= steps; d++) {
+      if (d && t3 < 0) break;
+      for (int b = 0; c + 3 * d + 2 * b <= steps; b++) {
+        const int left = steps - c - 3 * d - 2 * b;
+        if (left % 4 || (left && t4 < 0)) continue;
+        const int a = left / 4;
+        if ((a + b + c + d) % 2 == 0) continue;
+        const double t = a * t4 + d * t3 + b * t2 + c * t1;
+        if (t < best) {
+          best = t;
+          plan->count[4] = a;
+          plan->count[3] = d;
+          plan->count[2] = b;
+          plan->count[1] = c;
+        }
       }
     }
-  return plan->fours + plan->twos > 0;
+  return plan->passes() > 0;
 }
 
 static psb_status run_pipe(MapImpl **ms, const PipePlan &plan, int64_t *launches) {
@@ -403,16 +413,16 @@ static psb_status run_pipe(MapImpl **ms, const PipePlan &plan, int64_t *launches
   const bool per = ms[0]->kernel_id == PSB_KERNEL_DIFFUSION7_PERIODIC;
   GridImpl *g[2] = {ms[0]->grids[0], ms[0]->grids[1]};
   int at = 0;  // the grid that holds the state
-  for (int i = 0; i < plan.fours + plan.twos; i++) {
+  for (int i = 0; i < plan.passes(); i++) {
+    const int ns = i < plan.count[4] ? 4 : i < plan.count[4] + plan.count[3] ? 3 : 2;
     GridImpl *in = g[at], *out = g[at ^ 1];
     if (per && in->ghost_valid != PSB_BOUNDARY_PERIODIC && in->ghost_valid != kGhostXY)
       PSB_CHECK(launch_halo_fill(in, PSB_BOUNDARY_PERIODIC, r.stream));
-    PSB_CHECK(diff7_pipe_launch(*ms[0], in, out, i < plan.fours ? plan.four : plan.two, r.stream,
-                                launches));
+    PSB_CHECK(diff7_pipe_launch(*ms[0], in, out, plan.pass[ns], r.stream, launches));
     out->ghost_valid = per ? kGhostXY : PSB_BOUNDARY_NONE;
     at ^= 1;
   }
-  for (int i = 0; i <= plan.singles; i++) {
+  for (int i = 0; i <= plan.count[1]; i++) {
     PSB_CHECK(prepare_ghosts(*ms[at]));
     PSB_CHECK(launch_map(*ms[at], -1, launches));
     at ^= 1;

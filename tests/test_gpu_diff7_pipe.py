@@ -64,6 +64,18 @@ def test_passes_equal_single_steps(shape, dtype, periodic, fma):
         ps.set_fp_mode(ps.FP_EXACT)
 
 
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+def test_every_mix_of_passes(dtype):
+    """Step counts whose plans mix passes of four, three and two steps."""
+    ps.PSInit()
+    shape = (130, 97, 64)
+    for iters in (4, 5, 7, 8, 10):
+        got = _run(shape, dtype, False, iters, True)
+        want = _run(shape, dtype, False, iters, False)
+        assert got[2] < 2 * iters
+        assert U.bits_equal(got[0], want[0]) and U.bits_equal(got[1], want[1]), iters
+
+
 def test_large_runs_are_fused():
     """At 128^3 a run of 40 steps runs passes (fewer launches than steps)."""
     ps.PSInit()
