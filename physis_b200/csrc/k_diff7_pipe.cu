@@ -182,7 +182,7 @@ PipeConfig diff7_pipe_choose(int ns, bool dbl, bool per, bool fast, const int *n
     for (int shift = 3; shift <= 5; shift++)
       for (int threads = 64; threads <= (ns > 2 ? 384 : 192); threads += 32) {
         if (threads % (1 << shift)) continue;
-        for (int nc = 1; nc <= std::max(1, n[2] / 4) && nc <= 64; nc++) {
+        for (int nc = 1; nc <= std::max(1, n[2] / 2) && nc <= 128; nc++) {
           const PipeConfig c{ns, ns > 2 ? 2 : 4, threads, shift, (n[2] + nc - 1) / nc, 4};
           const double t = pipe_cost(c, dbl, per, fast, n);
           if (t > 0 && (best_cost < 0 || t < best_cost)) {
