@@ -911,6 +911,11 @@ static MemberTune member_tune(const BatchMemberHost &h) {
 // cubes of 128 and 256 gain 11% and 5%; cubes of 32, 48, 64 and 96 lose
 // 39%, 12%, 10% and 18% (small members get short z chunks, so each pass
 // re-reads a larger share of halo planes; 96 wastes 27% of its tile columns).
+// With 16-byte pressure loads (HimenoRows) one sweep gained more: cubes of 112
+// to 160 now run 1 to 27% faster with it, 192 to 384 within 12% either way,
+// and a batch with one member on the two-sweep list beside others on the
+// one-sweep list took 4.24 ms against 3.18; the shipped table therefore keeps
+// one sweep up to buckets of 256.
 static int default_sweeps(const BatchMemberHost &h) {
   const int *n = h.grids[0]->pub.dim;
   const int ix = n[0] - 2, iy = n[1] - 2, iz = n[2] - 2;
