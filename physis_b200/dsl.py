@@ -654,15 +654,22 @@ struct __psb_rgrid {
   int *bad;
 };
 
+// Whether index i, d from a point inside the grid, lies outside [0, n). One
+// step away there is one such index, and the comparison is the one a function
+// makes at its faces (x == 0, x == nx - 1): under such a condition the compiler
+// drops it.
+__device__ __forceinline__ bool __psb_outside(int d, int i, int n) {
+  return d == 0 ? false : d == -1 ? i == -1 : d == 1 ? i == n : (unsigned)i >= (unsigned)n;
+}
+
 template <typename T, class L, bool CX, bool CY, bool CZ>
 __device__ __forceinline__ T __psb_get(const __psb_rgrid<T, L, CX, CY, CZ> &g, int i, int j = 0,
                                        int k = 0) {
   const int dx = i - g.x, dy = j - g.y, dz = k - g.z;
   const T val = g.rows[L::id(g.slot, g.r, dy, dz)].e[2 + dx + g.v];
   if (!CX && !CY && !CZ) return val;
-  const bool out = (CX & (dx != 0) & ((unsigned)i >= (unsigned)g.n0)) |
-                   (CY & (dy != 0) & ((unsigned)j >= (unsigned)g.n1)) |
-                   (CZ & (dz != 0) & ((unsigned)k >= (unsigned)g.n2));
+  const bool out = (CX & __psb_outside(dx, i, g.n0)) | (CY & __psb_outside(dy, j, g.n1)) |
+                   (CZ & __psb_outside(dz, k, g.n2));
   *g.bad |= (int)out;
   return out ? T(0) : val;
 }
@@ -1032,6 +1039,8 @@ struct __psb_prog_{n} {{
           {known_x}
         }} else if (X == 0 && (x < at.lo0 || x >= at.hi0)) {{
           continue;
+        }} else if (C && X == 1) {{  // the domain lies inside every grid read
+          {known_x1}
         }}
         {handles}
         {n}__staged(x, y, z, {args});
@@ -1116,7 +1125,10 @@ extern "C" psb_status psb_dsl_staged_checked_{n}(const void *maps, const void *t
            minb=3 if few else 2, handles="\n        ".join(handles), args=", ".join(args),
            in_x=" && ".join(inside["x"]), in_yz=" && ".join(inside["y"] + inside["z"]),
            known_x="\n          ".join(known["x"]), known_y="\n        ".join(known["y"]),
-           known_z="\n      ".join(known["z"]))
+           known_z="\n      ".join(known["z"]), known_x1="\n          ".join(
+               ["__builtin_assume(at.x >= 0);", "__builtin_assume(x >= %s);" % "v"] +
+               ["__builtin_assume(x < tab.slot_dims[%d][0]);" % slot
+                for slot in sorted(info.staged_reads) if slot != info.emit_slot]))
 
 
 def _read_ranges(info):
