@@ -746,7 +746,7 @@ psb_status psb_batch_autotune(psb_batch *b, int force);
  * _DIFFUSION7_PERIODIC or _HIMENO19), type PS_FLOAT, and the member's size
  * bucket (each extent rounded up to a power of two, at least 8). A run
  * uses tile_x (consumer threads along x = tile_x / 4) and, for Himeno,
- * t_depth (2: two sweeps per pass of 64 x 8 tiles); the z chunk follows the
+ * t_depth (2: two sweeps per pass of 64 x 12 tiles); the z chunk follows the
  * batch's own rule. Setting an entry by hand pins the shape of a bucket. */
 #define PSB_BATCH_TUNE_BASE 100
 psb_status psb_batch_free(psb_batch *b);

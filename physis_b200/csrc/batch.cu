@@ -543,19 +543,20 @@ __global__ void __launch_bounds__(kBThreads, GROUP == 0 ? 3 : 2) k_batch(BatchDe
 // A member's local steps are cut into passes of one or two sweeps
 // (pass_start); a pass never straddles a residual check (a check step is
 // always the last step of its pass), so a check sees the sweep it needs.
-// Items are (member, pass, 64 x 8 tile x z chunk); the work list is ordered
+// Items are (member, pass, 64 x 12 tile x z chunk); the work list is ordered
 // by pass, then member, then tile, and an item depends on pass - 1 of its
 // member exactly as a single-sweep item depends on step - 1 (wait_item_deps:
 // the two-sweep halo of 2 cells stays inside the 27 tiles around it). Each
 // pass flips which buffer holds the state (buf[(cur0 + pass) & 1] in,
 // buf[(cur0 + pass + 1) & 1] out), so a two-sweep pass never writes the
-// buffer it reads. A CTA is one producer thread, five first-sweep warps and
-// four second-sweep warps on the rings of k_himeno_tb2.cuh; a one-sweep
+// buffer it reads. A CTA is one producer thread, seven first-sweep warps, six
+// second-sweep warps and the edge warp on the rings of k_himeno_tb2.cuh; a one-sweep
 // pass runs the same rings with the second stage storing the first sweep.
-// Every consumer warp completes one unit per item (nine per item).
+// Every consumer warp completes one unit per item (thirteen per item;
+// the edge warp none).
 // ---------------------------------------------------------------------------
 constexpr int kT2Units = kHtW1 + kHtW2;
-constexpr int kT2Threads = 32 * (1 + kT2Units);
+constexpr int kT2Threads = 32 * (1 + kT2Units + 1);  // and the edge warp
 constexpr int kT2SmemRing = 1024;
 constexpr size_t kT2Smem = 128 + kT2SmemRing + kHtRingBytes;
 
@@ -566,7 +567,7 @@ __device__ __forceinline__ bool pass_checked(const BMember &M, int q) {
   return is_check_step<1>(M, M.step0 + pass_end(M, q) - 1);
 }
 
-// Geometry of item t of a group-2 member: 64 x 8 tiles over the interior.
+// Geometry of item t of a group-2 member: 64 x 12 tiles over the interior.
 __device__ __forceinline__ void t2_geom(const BMember &M, int t, int &x0, int &y0, int &zb,
                                         int &nzl) {
   const int tile_x = t % M.tiles_x;
@@ -636,7 +637,7 @@ __device__ void t2_produce(const BatchDev &B, int step, const HtRings &R, uint64
   }
 }
 
-// Completion of a group-2 item by consumer warp cw (0..8): its FP64
+// Completion of a group-2 item by consumer warp cw (0..12): its FP64
 // residual partial when the pass ends with a check, one unit of the tile's
 // and of the pass's counter; the warp that completes the pass combines the
 // partials in index order, decides, and only then releases the pass.
@@ -709,9 +710,11 @@ __device__ void t2_consume(const BatchDev &B, const HtRings &R, uint64_t *qfull,
       int x0, y0, zb, nzl;
       t2_geom(M, dt, x0, y0, zb, nzl);
       bool ok;
-      if (first) {
-        ok = ht_stage1_tile(R, p1, pc, p2, threadIdx.x - 32, lane, M.dom, M.omega, x0, y0, zb,
-                            nzl, check && len == 1, &a);
+      if (cw == kT2Units) {
+        ok = ht_edge_tile<false>(R, p1, pc, p2, lane, M.dom, M.omega, x0, y0, zb, nzl);
+      } else if (first) {
+        ok = ht_stage1_tile<false>(R, p1, pc, p2, threadIdx.x - 32, lane, M.dom, M.omega, x0, y0,
+                                   zb, nzl, check && len == 1, &a);
       } else {
         const int par = (M.cur0 + ds) & 1;
         ok = ht_stage2_tile(R, p2, pc, threadIdx.x - 32 - 32 * kHtW1, lane,
@@ -723,12 +726,14 @@ __device__ void t2_consume(const BatchDev &B, const HtRings &R, uint64_t *qfull,
         return;
       }
     }
-    t2_item_done(M, ds, dt, cw, lane, check, check && !skip, a);
+    // The edge warp's points reach the output through the second-sweep warps,
+    // which complete the item.
+    if (cw < kT2Units) t2_item_done(M, ds, dt, cw, lane, check, check && !skip, a);
   }
 }
 
 // The group-2 kernel. step < 0: persistent (mode 0); step >= 0: item
-// blockIdx.x of that pass (mode 1). One CTA per SM (its rings take 175 KB).
+// blockIdx.x of that pass (mode 1). One CTA per SM (its rings take 223 KB).
 __global__ void __launch_bounds__(kT2Threads, 1) k_batch_tb2(BatchDev B, int step) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
   unsigned char *smem = aligned_smem(smem_raw);
@@ -740,7 +745,7 @@ __global__ void __launch_bounds__(kT2Threads, 1) k_batch_tb2(BatchDev B, int ste
     ht_init(R);
     for (int q = 0; q < kQ; q++) {
       mbar_init(&qfull[q], 1);
-      mbar_init(&qempty[q], kT2Units);
+      mbar_init(&qempty[q], kT2Units + 1);
     }
     mbar_fence_init();
   }
@@ -1035,8 +1040,8 @@ static HimenoGeom batch_hgeom(const GridImpl *g, int zc_floor, const MemberTune 
   return geo;
 }
 
-// Group 2: 64 x 8 tiles over the interior [1, n-1), x from 0; the pressure
-// box (72 x 12) is the tensor-map box of the member's p grids.
+// Group 2: 64 x 12 tiles over the interior [1, n-1), x from 0; the pressure
+// box (72 x 16) is the tensor-map box of the member's p grids.
 static HimenoGeom batch_t2geom(const GridImpl *g, int zc_floor, const MemberTune &mt) {
   HimenoGeom geo;
   geo.tx_threads = kHtTX / 4;
@@ -1746,7 +1751,7 @@ static psb_status batch_tune_member(const BatchMemberHost &h, psb_tune_config *b
   double best = -1, rule_ms = -1;
   // The rule is the batch's default: the fewest-tiles shape with the
   // default sweeps per pass. Himeno buckets also try the other depth (two
-  // sweeps: 64 x 8 tiles, recorded as tile_x 64).
+  // sweeps: 64 x 12 tiles, recorded as tile_x 64).
   const int rule_td = h.kind == BK_HIMENO ? default_sweeps(h) : 1;
   std::vector<std::array<int, 2>> cands;  // (tile width in threads or 0, t_depth)
   cands.push_back({0, rule_td});

@@ -101,7 +101,8 @@ struct Runtime {
   cudaStream_t stream = nullptr;
   cudaEvent_t ev_start = nullptr, ev_stop = nullptr;
   cudaEvent_t ev_join = nullptr;  // orders the runtime stream with the legacy stream
-  int *d_error = nullptr;     // device error word (timeouts)
+  int *d_error = nullptr;     // device error word (timeouts); [1] reads outside a grid, [2] rim_run
+  int rim_run = 0;            // himeno_rim_copy calls; d_error[2]: the last that found a difference
   psb_status last_status = PSB_OK;
   char last_error[256] = {0};  // text of the last CUDA failure
   int impl = PSB_IMPL_AUTO;
@@ -167,6 +168,9 @@ psb_status launch_halo_fill(GridImpl *g, int mode, cudaStream_t s);
 // Pitched 3-D grids in a stream-ordered memory pool (serving): allocation and
 // zero fill on stream s, free after the work queued on s.
 size_t grid_pitched_bytes(int elm_size, const int *dims);
+// The runtime's work grid in g's shape and layout (contents unspecified), for use
+// on its stream under its lock; nullptr where the memory is short.
+GridImpl *grid_work(const GridImpl *g);
 psb_status grid_alloc_pool(int type, const int *dims, cudaMemPool_t pool, cudaStream_t s,
                            GridImpl **out);
 void grid_free_pool(GridImpl *g, cudaStream_t s);
@@ -198,8 +202,11 @@ psb_status diff7_pipe_launch(MapImpl &m, GridImpl *in, GridImpl *out, const Pipe
 PipeConfig diff7_pipe_choose(int ns, bool dbl, bool per, bool fast, const int *n, double *cost);
 bool himeno_tb2_pair(MapImpl **ms, int n);
 int himeno_tb2_chunk(const __PSDomain &dom);  // z chunk of the pass over a domain
+// The cells around map m's domain from its input grid to dst, compared with its
+// output grid's on the way (Runtime::rim_run).
+psb_status himeno_rim_copy(const MapImpl &m, GridImpl *dst, cudaStream_t s, int64_t *launches);
 psb_status himeno_tb2_launch(MapImpl &m1, MapImpl &m2, GridImpl *in, GridImpl *out,
-                             int zchunk, cudaStream_t s, int64_t *launches);
+                             int zchunk, bool rims, cudaStream_t s, int64_t *launches);
 psb_status generic_tma_launch(MapImpl &m, const GenericDesc &gd, int color, cudaStream_t s,
                               int64_t *launches);
 void generic_note_impl(int impl);

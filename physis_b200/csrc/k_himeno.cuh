@@ -78,6 +78,43 @@ struct HimenoRows {
   }
 };
 
+// The same for V points (4, or 1 with offsets of any alignment), kept from plane
+// to plane: of each turn's nine rows only the three of plane z+1 are loaded, the
+// others are the last turn's, and a plane is read once, in the turn it arrives.
+template <int V>
+struct HimenoWalk {
+  float mn[V], m[V + 2], ms[V];              // plane z-1: y-1, y, y+1
+  float cn[V + 2], c[V + 2], cs[V + 2];      // plane z
+  float pn[V + 2], p[V + 2], ps[V + 2];      // plane z+1
+
+  static __device__ __forceinline__ void row(const float *q, float (&e)[V + 2]) {
+    if constexpr (V == 4) {
+      HimenoRows::row6(q, e);
+    } else {
+#pragma unroll
+      for (int v = 0; v < V + 2; v++) e[v] = q[v - 1];
+    }
+  }
+  __device__ __forceinline__ void load(const float *q, int o, int BX) {
+    row(q + o - BX, pn);
+    row(q + o, p);
+    row(q + o + BX, ps);
+  }
+  // Plane z+1 becomes plane z.
+  __device__ __forceinline__ void step() {
+#pragma unroll
+    for (int v = 0; v < V; v++) mn[v] = cn[1 + v], ms[v] = cs[1 + v];
+#pragma unroll
+    for (int v = 0; v < V + 2; v++) m[v] = c[v], cn[v] = pn[v], c[v] = p[v], cs[v] = ps[v];
+  }
+  // Point v with its coefficients (himeno_point).
+  __device__ __forceinline__ float point(const float *co, int v, float omega, float *ss) const {
+    return himeno_point(co, c[1 + v], c[2 + v], c[v], cs[1 + v], cn[1 + v], p[1 + v], m[1 + v],
+                        ps[1 + v], pn[1 + v], ms[v], mn[v], cs[2 + v], cn[2 + v], cs[v], cn[v],
+                        p[2 + v], m[2 + v], p[v], m[v], omega, ss);
+  }
+};
+
 struct HimenoGeom {
   int ax0, ay0, az0;
   int tiles_x, tiles_y, zchunk, stages, bx, by, stage_bytes, x_base;

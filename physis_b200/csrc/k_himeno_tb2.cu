@@ -6,19 +6,24 @@
 // each coefficient once: per CTA and tile, a producer thread streams the
 // input pressure planes (box TX+8 x TY+4: the tile with a 2-cell halo,
 // x rounded out to 16 bytes) into ring R1 and the twelve coefficient planes
-// of the tile with a 1-cell halo (box TX+8 x TY+2) into ring RC; five
-// "stage-1" warps compute the first sweep over the tile plus a 1-cell halo
-// (the points the second sweep reads) into ring R2, whose stages are laid
-// out like the coefficient boxes; four "stage-2" warps compute the second
-// sweep of the tile from R2 and the same coefficient stages and store it.
+// of the tile with a 1-cell halo (box TX+8 x TY+2) into ring RC; seven
+// "stage-1" warps and one for the halo columns compute the first sweep over
+// the tile plus a 1-cell halo (the points the second sweep reads) into ring
+// R2, whose stages are laid out like the coefficient boxes; six "stage-2"
+// warps compute the second sweep of the tile from R2 and the same coefficient
+// stages and store it.
 // Per output pair of updates the pass moves 4 B of p in, 4 B out and 48 B
 // of coefficients (with the halo columns and rows of neighbouring tiles
 // mostly from L2): about half the bytes of two single sweeps.
 //
 // Every point of both sweeps uses the single-sweep arithmetic
 // (himeno_point, round-to-nearest, the C evaluation order), and first-sweep
-// values outside the domain are the input values (the sweep never writes
-// them), so the result equals two single sweeps bit for bit. The residual
+// values outside the domain are those of the grid the first sweep writes (it
+// leaves them there), so the result equals two single sweeps bit for bit, also
+// where the two grids' rims differ: a run keeps that grid untouched until its
+// last two sweeps and alternates between the input and the work grid, whose
+// rim is the input's (himeno_rim_copy, which also finds out whether the rims
+// differ at all). The residual
 // sum of ss*ss of each sweep is accumulated over the tile's own points in
 // FP64 and combined per sweep in a fixed order (one partial per CTA, the
 // last CTA adds them in index order) into the history of the map whose
@@ -27,13 +32,14 @@
 // Persistent: one CTA per SM walks the (tile, z chunk) items blockIdx.x,
 // blockIdx.x + gridDim.x, ...; its rings carry on from item to item.
 #include <algorithm>
+#include <climits>
 #include <cstring>
 
 #include "k_himeno_tb2.cuh"
 
 namespace psb {
 
-constexpr int kHtThreads = 32 + 32 * (kHtW1 + kHtW2);
+constexpr int kHtThreads = 32 + 32 * (kHtW1 + kHtW2 + 1);
 constexpr int kHtSmemRing = 1024;  // barriers, scratch and flags before the rings
 constexpr int kHtSmem = 128 + kHtSmemRing + kHtRingBytes;
 
@@ -45,6 +51,9 @@ struct HtGeom {
   int ax0, ay0, az0;  // tensor coordinates of logical (0,0,0)
   int tiles_x, tiles_y, nzc, zchunk;
   int64_t items;
+  HtRim rim;
+  const int *rim_differs;  // == rim_run: rim is not the input's (himeno_rim_copy)
+  int rim_run;
 };
 
 __global__ void __launch_bounds__(kHtThreads, 1)
@@ -95,12 +104,27 @@ __global__ void __launch_bounds__(kHtThreads, 1)
 
   double acc = 0.0;
   bool bad = false;
+  const bool rim = *hg.rim_differs == hg.rim_run;
+  if (warp > kHtW1 + kHtW2) {
+    RingPos p1{0, 0}, pc{0, 0}, p2{0, 0};
+    for (int64_t item = blockIdx.x; item < hg.items && !bad; item += gridDim.x) {
+      int x0, y0, zb, nzl;
+      item_geom(item, x0, y0, zb, nzl);
+      bad = rim ? !ht_edge_tile<true>(R, p1, pc, p2, lane, d, omega, x0, y0, zb, nzl, hg.rim)
+                : !ht_edge_tile<false>(R, p1, pc, p2, lane, d, omega, x0, y0, zb, nzl);
+    }
+    if (bad && lane == 0) atomicExch(err, 1);
+    return;
+  }
   if (warp <= kHtW1) {
     RingPos p1{0, 0}, pc{0, 0}, p2{0, 0};
     for (int64_t item = blockIdx.x; item < hg.items && !bad; item += gridDim.x) {
       int x0, y0, zb, nzl;
       item_geom(item, x0, y0, zb, nzl);
-      bad = !ht_stage1_tile(R, p1, pc, p2, tid - 32, lane, d, omega, x0, y0, zb, nzl, true, &acc);
+      bad = rim ? !ht_stage1_tile<true>(R, p1, pc, p2, tid - 32, lane, d, omega, x0, y0, zb, nzl,
+                                        true, &acc, hg.rim)
+                : !ht_stage1_tile<false>(R, p1, pc, p2, tid - 32, lane, d, omega, x0, y0, zb, nzl,
+                                         true, &acc);
     }
   } else {
     RingPos p2{0, 0}, pc{0, 0};
@@ -230,10 +254,59 @@ static psb_status ht_residual(MapImpl &m, int nblocks, Residual *r) {
   return PSB_OK;
 }
 
+// The cells around the domain (one deep, with edges and corners), src -> dst;
+// *differs = run where other holds another value in one of them.
+__global__ void k_himeno_rim(const float *src, const float *other, float *dst, int64_t sy,
+                             int64_t sz, Dom3 d, int *differs, int run) {
+  const int ex = d.hi[0] - d.lo[0] + 2, ey = d.hi[1] - d.lo[1] + 2, ez = d.hi[2] - d.lo[2] + 2;
+  const int64_t nz = (int64_t)ex * ey, ny = (int64_t)ex * ez, nx = (int64_t)ey * ez;
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < 2 * (nx + ny + nz);
+       i += (int64_t)gridDim.x * blockDim.x) {
+    int x, y, z;
+    if (i < 2 * nz) {
+      const int64_t k = i % nz;
+      x = (int)(k % ex), y = (int)(k / ex), z = i < nz ? 0 : ez - 1;
+    } else if (i < 2 * (nz + ny)) {
+      const int64_t k = (i - 2 * nz) % ny;
+      x = (int)(k % ex), z = (int)(k / ex), y = i - 2 * nz < ny ? 0 : ey - 1;
+    } else {
+      const int64_t k = (i - 2 * (nz + ny)) % nx;
+      y = (int)(k % ey), z = (int)(k / ey), x = i - 2 * (nz + ny) < nx ? 0 : ex - 1;
+    }
+    const int64_t o = (x + d.lo[0] - 1) + (y + d.lo[1] - 1) * sy + (z + d.lo[2] - 1) * sz;
+    const float v = src[o];
+    dst[o] = v;
+    if (__float_as_int(v) != __float_as_int(other[o])) *differs = run;
+  }
+}
+
+psb_status himeno_rim_copy(const MapImpl &m, GridImpl *dst, cudaStream_t s, int64_t *launches) {
+  Runtime &r = rt();
+  const GridImpl *src = m.grids[0], *other = m.grids[1];
+  r.rim_run = r.rim_run == INT_MAX ? 1 : r.rim_run + 1;
+  Dom3 d;
+  int64_t e[3];
+  for (int i = 0; i < 3; i++) {
+    d.lo[i] = m.dom.local_min[i];
+    d.hi[i] = m.dom.local_max[i];
+    e[i] = d.hi[i] - d.lo[i] + 2;
+  }
+  const int64_t n = 2 * (e[0] * e[1] + e[0] * e[2] + e[1] * e[2]);
+  k_himeno_rim<<<(unsigned)std::min<int64_t>((n + 255) / 256, 8 * r.sm_count), 256, 0, s>>>(
+      (const float *)src->view().origin, (const float *)other->view().origin,
+      (float *)dst->view().origin, src->sy, src->sz, d, r.d_error + 2, r.rim_run);
+  (*launches)++;
+  PSB_TRY(cudaGetLastError());
+  return PSB_OK;
+}
+
 // Two sweeps, in -> out: the first is map m1's sweep, the second m2's (their
-// residuals go to their histories when both maps have them enabled).
+// residuals go to their histories when both maps have them enabled). in holds
+// the rim of m1's input grid; the rim of m1's output grid is read, not written.
+// rims: himeno_rim_copy ran for these maps (else both grids' rims are taken to
+// be the same).
 psb_status himeno_tb2_launch(MapImpl &m1, MapImpl &m2, GridImpl *in, GridImpl *out,
-                             int zchunk, cudaStream_t s, int64_t *launches) {
+                             int zchunk, bool rims, cudaStream_t s, int64_t *launches) {
   Runtime &r = rt();
   const CUtensorMap *pmap = nullptr;
   PSB_CHECK(get_tmap(in, kHtBX, kHtBY1, &pmap));
@@ -255,6 +328,10 @@ psb_status himeno_tb2_launch(MapImpl &m1, MapImpl &m2, GridImpl *in, GridImpl *o
     d.hi[i] = m1.dom.local_max[i];
   }
   HtGeom hg;
+  const GridImpl *B = m1.grids[1];
+  hg.rim = HtRim{(const float *)B->view().origin, B->sy, B->sz, B->pub.dim[0], B->pub.dim[1]};
+  hg.rim_differs = r.d_error + 2;
+  hg.rim_run = rims ? r.rim_run : -1;
   hg.ax0 = in->pad_left;
   hg.ay0 = in->halo;
   hg.az0 = in->halo;

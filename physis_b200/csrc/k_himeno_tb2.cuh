@@ -5,37 +5,53 @@
 // (all in one CTA's shared memory, positions carried from tile to tile):
 //  R1  input pressure planes, box TX+8 x TY+4 (the tile with a 2-cell halo,
 //      x from x0-4 so the box starts on 16 bytes); one producer arrival,
-//      one release per stage-1 warp;
+//      one release per stage-1 and edge warp;
 //  RC  the twelve coefficient boxes of a plane, TX+8 x TY+2 (a 1-cell
 //      halo), field f at f * kHtField; one producer arrival, one release
-//      per stage-1 and per stage-2 warp;
+//      per stage-1, edge and stage-2 warp;
 //  R2  first-sweep planes over the tile and its 1-cell halo, laid out like
-//      one coefficient box; one arrival per stage-1 warp, one release per
-//      stage-2 warp.
-// Stage 1 (5 warps) computes the first sweep over (TX+2) x (TY+2) points
-// per plane (64-point rows as float4 vectors, the two halo columns as 20
-// scalar points); points outside the domain keep the input value, as a
-// sweep that never writes them would. Stage 2 (4 warps) computes the second
-// sweep of the tile from R2 and stores it, or (copy) stores the first sweep
-// itself, which makes a one-sweep pass of the same rings. Both use the
-// single-sweep arithmetic (himeno_point), so results equal single sweeps
-// bit for bit.
+//      one coefficient box; one arrival per stage-1 and edge warp, one
+//      release per stage-2 warp.
+// Stage 1 (7 warps) and the edge warp compute the first sweep over (TX+2) x
+// (TY+2) points per plane: stage 1 the 64-point rows as float4 vectors, the
+// edge warp the two halo columns, 28 scalar points; points outside the domain
+// take the value that the grid written by the first sweep holds there (HtRim),
+// or the input's where they are known to be the same. Stage 2 (6
+// warps) computes the second sweep of the tile from R2 and stores it, or (copy)
+// stores the first sweep itself, which makes a one-sweep pass of the same
+// rings. Both use the single-sweep arithmetic (himeno_point), so results equal
+// single sweeps bit for bit.
+//
+// What bounds it: one CTA fits an SM, so loads and warps in flight are scarce.
+// Every warp holds the planes around its points in registers and reads each
+// plane and coefficient stage once, first thing in the turn, and releases it
+// there: the rings are then prefetch only, and shared memory carries 84
+// wavefronts per warp and plane instead of 124. The halo columns have a warp of
+// their own (as lanes of the stage-1 warps they added a point's chain to the
+// slower stage), and what shared memory the rings gave up went into twelve rows
+// per tile, which read 1.17 coefficient rows per row instead of 1.25.
+// 257 x 257 x 513, us per sweep: 272 with eight rows and planes read from the
+// rings; 253 with the edge warp; 232 with the planes in registers; 208 released
+// early, 202 with five coefficient stages; 184 with twelve rows (0.78 of the
+// measured peak for the pass's 28 B per update). Fourteen rows need 17 warps,
+// which leaves 96 registers and spills (458); two points a thread instead of
+// four changes nothing; x neighbours by shuffle cost 8% (a longer chain).
 #pragma once
 
 #include "k_himeno.cuh"
 
 namespace psb {
 
-constexpr int kHtTX = 64, kHtTY = 8, kHtV = 4;
+constexpr int kHtTX = 64, kHtTY = 12, kHtV = 4;
 constexpr int kHtBX = kHtTX + 8;           // every box: x from x0 - 4
 constexpr int kHtBY1 = kHtTY + 4;          // input p: y from y0 - 2
 constexpr int kHtBY2 = kHtTY + 2;          // first sweep and coefficients: y from y0 - 1
 // Ring depths (stages) of R1, R2 and RC; build options for measurement.
 #ifndef PSB_HT_S1
-#define PSB_HT_S1 6
+#define PSB_HT_S1 4
 #endif
 #ifndef PSB_HT_S2
-#define PSB_HT_S2 4
+#define PSB_HT_S2 3
 #endif
 #ifndef PSB_HT_SC
 #define PSB_HT_SC 4
@@ -46,10 +62,13 @@ constexpr int kHtStage1 = (kHtBX * kHtBY1 * 4 + 127) / 128 * 128;
 constexpr int kHtStage2 = (kHtBX * kHtBY2 * 4 + 127) / 128 * 128;
 constexpr int kHtField = kHtStage2;        // one coefficient box
 constexpr int kHtStageC = 12 * kHtField;
-constexpr int kHtW1 = 5, kHtW2 = 4;        // stage-1 and stage-2 warps
+constexpr int kHtW1 = kHtTX / kHtV * (kHtTY + 2) / 32;  // stage-1 warps
+constexpr int kHtW2 = kHtTX / kHtV * kHtTY / 32;        // stage-2 warps; one edge warp more
+constexpr int kHtEdge = 2 * (kHtTY + 2);   // points of the two halo columns
 constexpr int kHtRingBytes = kHtS1 * kHtStage1 + kHtS2 * kHtStage2 + kHtSC * kHtStageC;
 static_assert(kHtTX / kHtV * (kHtTY + 2) == 32 * kHtW1, "stage-1 threads cover the halo rows");
 static_assert(kHtTX / kHtV * kHtTY == 32 * kHtW2, "stage-2 threads cover the tile");
+static_assert(kHtEdge <= 32, "one edge point per lane");
 
 struct HtRings {
   uint64_t *f1, *e1, *f2, *e2, *fc, *ec;  // full/empty barriers (8 slots each)
@@ -74,27 +93,16 @@ __device__ __forceinline__ HtRings ht_rings(uint64_t *bars, unsigned char *rings
 __device__ __forceinline__ void ht_init(const HtRings &R) {
   for (int i = 0; i < kHtS1; i++) {
     mbar_init(&R.f1[i], 1);
-    mbar_init(&R.e1[i], kHtW1);
+    mbar_init(&R.e1[i], kHtW1 + 1);
   }
   for (int i = 0; i < kHtS2; i++) {
-    mbar_init(&R.f2[i], kHtW1);
+    mbar_init(&R.f2[i], kHtW1 + 1);
     mbar_init(&R.e2[i], kHtW2);
   }
   for (int i = 0; i < kHtSC; i++) {
     mbar_init(&R.fc[i], 1);
-    mbar_init(&R.ec[i], kHtW1 + kHtW2);
+    mbar_init(&R.ec[i], kHtW1 + 1 + kHtW2);
   }
-}
-
-// 19 pressure values around offset o of three planes with row length kHtBX
-// (m: z-1, c: z, p: z+1) and the point's 12 coefficients.
-__device__ __forceinline__ float ht_point(const float *co, const float *qm, const float *qc,
-                                          const float *qp, int o, float omega, float *ss) {
-  constexpr int B = kHtBX;
-  return himeno_point(co, qc[o], qc[o + 1], qc[o - 1], qc[o + B], qc[o - B], qp[o], qm[o],
-                      qp[o + B], qp[o - B], qm[o + B], qm[o - B], qc[o + 1 + B], qc[o + 1 - B],
-                      qc[o - 1 + B], qc[o - 1 - B], qp[o + 1], qm[o + 1], qp[o - 1], qm[o - 1],
-                      omega, ss);
 }
 
 __device__ __forceinline__ bool ht_wait(uint64_t *bar, uint32_t parity) {
@@ -147,98 +155,159 @@ __device__ __forceinline__ void ht_drain(const HtRings &R, RingPos p1, RingPos p
   ring_drain(Ring{R.fc, R.ec, R.rc, kHtSC, kHtStageC}, pc);
 }
 
-// Stage-1 warps (thread t in [0, 160)): the first sweep of one tile into R2.
-// Thread t owns 4 x points of halo row t / 16 (y = y0 - 1 + row); every
-// eighth thread also owns one of the 20 edge points (x0 - 1 and x0 + TX of
-// each row). With acc_on, the FP64 sum of ss*ss over the tile's own domain
-// points is added to *acc. False (warp-uniformly) if a bounded wait gave up.
+// The walk's first two planes, each released as soon as it is in registers.
+template <int V>
+__device__ __forceinline__ bool ht_begin(HimenoWalk<V> &h, RingPos &p, int S, uint64_t *full,
+                                         uint64_t *empty, const unsigned char *ring, int stage,
+                                         int ofs, int lane) {
+#pragma unroll
+  for (int i = 0; i < 2; i++) {
+    if (!ht_wait(&full[p.slot], p.round & 1)) return false;
+    h.step();
+    h.load(reinterpret_cast<const float *>(ring + p.slot * stage), ofs, kHtBX);
+    ht_release(&empty[p.slot], lane);
+    ring_next(p, S);
+  }
+  return true;
+}
+
+// Where first-sweep values outside the domain come from: the grid that the
+// first sweep writes, as a sweep leaves them there (p: logical (0,0,0); nx, ny:
+// points inside it).
+struct HtRim {
+  const float *p;
+  int64_t sy, sz;
+  int nx, ny;
+};
+
+// Stage-1 warps (thread t in [0, 224)): the first sweep of one tile into R2.
+// Thread t owns 4 x points of halo row t / 16 (y = y0 - 1 + row). Points
+// outside the domain take their value from rim (RIM; fetched to L1 at the head
+// of the turn, read at its end) or keep the input's. The two mostly are the same
+// and the loads cost 10 to 40%, so the caller chooses. With acc_on, the FP64 sum of
+// ss*ss over the tile's own domain points is added to *acc. False
+// (warp-uniformly) if a bounded wait gave up.
+template <bool RIM>
 __device__ __forceinline__ bool ht_stage1_tile(const HtRings &R, RingPos &p1, RingPos &pc,
                                                RingPos &p2, int t, int lane, const Dom3 d,
                                                float omega, int x0, int y0, int zb, int nzl,
-                                               bool acc_on, double *acc) {
+                                               bool acc_on, double *acc,
+                                               const HtRim rim = HtRim{}) {
   const int tx = t % (kHtTX / kHtV), row = t / (kHtTX / kHtV);
   const int cofs = row * kHtBX + 4 + tx * kHtV;        // R2 / RC offset of the vector
   const int pofs = (row + 1) * kHtBX + 4 + tx * kHtV;  // R1 offset of the vector
-  const bool edge = (t & 7) == 0;
-  const int e = t >> 3;                                // 0..19
-  const int ecol = e / (kHtTY + 2), erow = e % (kHtTY + 2);
-  const int ex_off = ecol ? 4 + kHtTX : 3;
-  const int ecofs = erow * kHtBX + ex_off, epofs = (erow + 1) * kHtBX + ex_off;
   const int xg = x0 + tx * kHtV, yg = y0 - 1 + row;
-  const int ex = ecol ? x0 + kHtTX : x0 - 1, ey = y0 - 1 + erow;
   const bool row_in = yg >= d.lo[1] && yg < d.hi[1];
   const bool row_own = row_in && row >= 1 && row <= kHtTY;
-  RingPos pm = p1, pz = p1;  // input planes z-1 and z
-  ring_next(pz, kHtS1);
-  RingPos pp = pz;
-  if (!ht_wait(&R.f1[pm.slot], pm.round & 1) || !ht_wait(&R.f1[pz.slot], pz.round & 1))
-    return false;
+  const bool xy_in = row_in && xg >= d.lo[0] && xg + kHtV <= d.hi[0];
+  // The vector's points in the rim grid (a row of a pitched grid ends on a
+  // whole vector).
+  const bool has_rim = RIM && xg < rim.nx && yg < rim.ny;
+  auto rim_at = [&](int z) { return rim.p + xg + (int64_t)yg * rim.sy + (int64_t)z * rim.sz; };
+  HimenoWalk<kHtV> h = {};
+  if (!ht_begin(h, p1, kHtS1, R.f1, R.e1, R.r1, kHtStage1, pofs, lane)) return false;
   double a = 0.0;
   for (int j = 0; j < nzl + 2; j++) {
     const int z = zb - 1 + j;
-    ring_next(pp, kHtS1);
-    if (!ht_wait(&R.f1[pp.slot], pp.round & 1) || !ht_wait(&R.fc[pc.slot], pc.round & 1))
-      return false;
-    const float *qm = reinterpret_cast<const float *>(R.r1 + pm.slot * kHtStage1);
-    const float *qc = reinterpret_cast<const float *>(R.r1 + pz.slot * kHtStage1);
-    const float *qp = reinterpret_cast<const float *>(R.r1 + pp.slot * kHtStage1);
-    const unsigned char *cs = R.rc + pc.slot * kHtStageC;
     const bool z_in = z >= d.lo[2] && z < d.hi[2];
+    if (has_rim && !(z_in && xy_in))
+      asm volatile("prefetch.global.L1 [%0];" ::"l"(rim_at(z)));
+    if (!ht_wait(&R.f1[p1.slot], p1.round & 1) || !ht_wait(&R.fc[pc.slot], pc.round & 1))
+      return false;
+    const unsigned char *cs = R.rc + pc.slot * kHtStageC;
+    Vec16<float> co[12];
+#pragma unroll
+    for (int f = 0; f < 12; f++)
+      co[f] = lds16(reinterpret_cast<const float *>(cs + f * kHtField) + cofs);
+    h.step();
+    h.load(reinterpret_cast<const float *>(R.r1 + p1.slot * kHtStage1), pofs, kHtBX);
+    ht_release(&R.e1[p1.slot], lane);
+    ht_release(&R.ec[pc.slot], lane);  // stage 2 holds its own claim on the stage
+    ring_next(p1, kHtS1);
+    ring_next(pc, kHtSC);
     const bool z_own = z_in && j >= 1 && j <= nzl;
     float outv[kHtV];
-    {
-      Vec16<float> co[12];
 #pragma unroll
-      for (int f = 0; f < 12; f++)
-        co[f] = lds16(reinterpret_cast<const float *>(cs + f * kHtField) + cofs);
-      HimenoRows h;
-      h.load(qm, qc, qp, pofs, kHtBX);
-#pragma unroll
-      for (int v = 0; v < kHtV; v++) {
-        const int x = xg + v;
-        float c[12];
-#pragma unroll
-        for (int f = 0; f < 12; f++) c[f] = co[f].v[v];
-        float ss;
-        const float r = h.point(c, v, omega, &ss);
-        const bool in = z_in && row_in && x >= d.lo[0] && x < d.hi[0];
-        outv[v] = in ? r : h.c[1 + v];
-        if (acc_on && in && z_own && row_own) a += (double)ss * (double)ss;
-      }
-    }
-    float eout = 0.f;
-    if (edge) {
+    for (int v = 0; v < kHtV; v++) {
+      const int x = xg + v;
       float c[12];
 #pragma unroll
-      for (int f = 0; f < 12; f++) c[f] = reinterpret_cast<const float *>(cs + f * kHtField)[ecofs];
+      for (int f = 0; f < 12; f++) c[f] = co[f].v[v];
       float ss;
-      const float r = ht_point(c, qm, qc, qp, epofs, omega, &ss);
-      const bool in = z_in && ey >= d.lo[1] && ey < d.hi[1] && ex >= d.lo[0] && ex < d.hi[0];
-      eout = in ? r : qc[epofs];
+      const float r = h.point(c, v, omega, &ss);
+      const bool in = z_in && row_in && x >= d.lo[0] && x < d.hi[0];
+      outv[v] = in || RIM ? r : h.c[1 + v];
+      if (acc_on && in && z_own && row_own) a += (double)ss * (double)ss;
     }
-    ht_release(&R.e1[pm.slot], lane);  // input plane z-1 is done
-    ht_release(&R.ec[pc.slot], lane);  // stage 2 holds its own claim on the stage
-    ring_next(pc, kHtSC);
+    if (has_rim && !(z_in && xy_in)) {
+      const float4 q = __ldg(reinterpret_cast<const float4 *>(rim_at(z)));
+      const float w[kHtV] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+      for (int v = 0; v < kHtV; v++)
+        if (!(z_in && row_in && xg + v >= d.lo[0] && xg + v < d.hi[0])) outv[v] = w[v];
+    }
     // The first-sweep plane z into the next stage of R2.
     if (p2.round > 0 && !ht_wait(&R.e2[p2.slot], (p2.round - 1) & 1)) return false;
     float *dst = reinterpret_cast<float *>(R.r2 + p2.slot * kHtStage2);
     *reinterpret_cast<float4 *>(dst + cofs) = make_float4(outv[0], outv[1], outv[2], outv[3]);
-    if (edge) dst[ecofs] = eout;
     ht_release(&R.f2[p2.slot], lane);
     ring_next(p2, kHtS2);
-    pm = pz;
-    pz = pp;
   }
-  // The last two input planes were never a plane z-1.
-  ht_release(&R.e1[pm.slot], lane);
-  ht_release(&R.e1[pz.slot], lane);
-  p1 = pz;
-  ring_next(p1, kHtS1);
   *acc += a;
   return true;
 }
 
-// Stage-2 warps (thread t in [0, 128)): the second sweep of the tile from R2
+// The edge warp: the first sweep's halo columns x0 - 1 and x0 + TX of one
+// tile into R2, lane e < 28 the point of row e % 14 of column e / 14; rim as in
+// stage 1. False (warp-uniformly) if a bounded wait gave up.
+template <bool RIM>
+__device__ __forceinline__ bool ht_edge_tile(const HtRings &R, RingPos &p1, RingPos &pc,
+                                             RingPos &p2, int lane, const Dom3 d, float omega,
+                                             int x0, int y0, int zb, int nzl,
+                                             const HtRim rim = HtRim{}) {
+  const int e = min(lane, kHtEdge - 1);
+  const int col = e / (kHtTY + 2), row = e % (kHtTY + 2);
+  const int xo = col ? 4 + kHtTX : 3;
+  const int cofs = row * kHtBX + xo, pofs = (row + 1) * kHtBX + xo;
+  const int x = col ? x0 + kHtTX : x0 - 1, y = y0 - 1 + row;
+  const bool in_xy = y >= d.lo[1] && y < d.hi[1] && x >= d.lo[0] && x < d.hi[0];
+  const float *rp = nullptr;
+  if (RIM && x >= 0 && x < rim.nx && y < rim.ny)
+    rp = rim.p + x + (int64_t)y * rim.sy + (int64_t)(zb - 1) * rim.sz;
+  HimenoWalk<1> h = {};
+  if (!ht_begin(h, p1, kHtS1, R.f1, R.e1, R.r1, kHtStage1, pofs, lane)) return false;
+  for (int j = 0; j < nzl + 2; j++) {
+    const int z = zb - 1 + j;
+    const bool in = in_xy && z >= d.lo[2] && z < d.hi[2];
+    float rv = 0.f;
+    if (RIM) {
+      if (!in && rp) rv = __ldg(rp);
+      if (rp) rp += rim.sz;
+    }
+    if (!ht_wait(&R.f1[p1.slot], p1.round & 1) || !ht_wait(&R.fc[pc.slot], pc.round & 1))
+      return false;
+    const unsigned char *cs = R.rc + pc.slot * kHtStageC;
+    float c[12];
+#pragma unroll
+    for (int f = 0; f < 12; f++) c[f] = reinterpret_cast<const float *>(cs + f * kHtField)[cofs];
+    h.step();
+    h.load(reinterpret_cast<const float *>(R.r1 + p1.slot * kHtStage1), pofs, kHtBX);
+    ht_release(&R.e1[p1.slot], lane);
+    ht_release(&R.ec[pc.slot], lane);
+    ring_next(p1, kHtS1);
+    ring_next(pc, kHtSC);
+    float ss;
+    const float r = h.point(c, 0, omega, &ss);
+    const float out = in ? r : RIM ? rv : h.c[1];
+    if (p2.round > 0 && !ht_wait(&R.e2[p2.slot], (p2.round - 1) & 1)) return false;
+    if (lane < kHtEdge) reinterpret_cast<float *>(R.r2 + p2.slot * kHtStage2)[cofs] = out;
+    ht_release(&R.f2[p2.slot], lane);
+    ring_next(p2, kHtS2);
+  }
+  return true;
+}
+
+// Stage-2 warps (thread t in [0, 192)): the second sweep of the tile from R2
 // and the coefficient stages of its planes, stored to pout (copy: the first
 // sweep itself is stored). Thread t owns 4 x points of tile row t / 16.
 // With acc_on (and not copy), the FP64 sum of ss*ss over the tile's domain
@@ -257,42 +326,37 @@ __device__ __forceinline__ bool ht_stage2_tile(const HtRings &R, RingPos &p2, Ri
   if (!ht_wait(&R.fc[pc.slot], pc.round & 1)) return false;
   ht_release(&R.ec[pc.slot], lane);
   ring_next(pc, kHtSC);
-  RingPos pm = p2, pz = p2;
-  ring_next(pz, kHtS2);
-  RingPos pp = pz;
-  if (!ht_wait(&R.f2[pm.slot], pm.round & 1) || !ht_wait(&R.f2[pz.slot], pz.round & 1))
-    return false;
+  HimenoWalk<kHtV> h = {};
+  if (!ht_begin(h, p2, kHtS2, R.f2, R.e2, R.r2, kHtStage2, ofs, lane)) return false;
   double a = 0.0;
   int64_t off = (int64_t)xg + (int64_t)yg * sy + (int64_t)zb * sz;
   for (int i = 0; i < nzl; i++) {
-    ring_next(pp, kHtS2);
-    if (!ht_wait(&R.f2[pp.slot], pp.round & 1) || !ht_wait(&R.fc[pc.slot], pc.round & 1))
-      return false;
-    const float *qm = reinterpret_cast<const float *>(R.r2 + pm.slot * kHtStage2);
-    const float *qc = reinterpret_cast<const float *>(R.r2 + pz.slot * kHtStage2);
-    const float *qp = reinterpret_cast<const float *>(R.r2 + pp.slot * kHtStage2);
+    // The coefficients are there before the first-sweep plane z+1 is.
+    if (!ht_wait(&R.fc[pc.slot], pc.round & 1)) return false;
     const unsigned char *cs = R.rc + pc.slot * kHtStageC;
+    Vec16<float> co[12];
+#pragma unroll
+    for (int f = 0; f < 12; f++)
+      co[f] = lds16(reinterpret_cast<const float *>(cs + f * kHtField) + ofs);
+    ht_release(&R.ec[pc.slot], lane);
+    ring_next(pc, kHtSC);
+    if (!ht_wait(&R.f2[p2.slot], p2.round & 1)) return false;
+    h.step();
+    h.load(reinterpret_cast<const float *>(R.r2 + p2.slot * kHtStage2), ofs, kHtBX);
+    ht_release(&R.e2[p2.slot], lane);
+    ring_next(p2, kHtS2);
     if (row_in) {
       float outv[kHtV];
-      if (copy) {
 #pragma unroll
-        for (int v = 0; v < kHtV; v++) outv[v] = qc[ofs + v];
-      } else {
-        Vec16<float> co[12];
+      for (int v = 0; v < kHtV; v++) {
+        float c[12];
 #pragma unroll
-        for (int f = 0; f < 12; f++)
-          co[f] = lds16(reinterpret_cast<const float *>(cs + f * kHtField) + ofs);
-        HimenoRows h;
-        h.load(qm, qc, qp, ofs, kHtBX);
-#pragma unroll
-        for (int v = 0; v < kHtV; v++) {
-          float c[12];
-#pragma unroll
-          for (int f = 0; f < 12; f++) c[f] = co[f].v[v];
-          float ss;
-          outv[v] = h.point(c, v, omega, &ss);
-          if (acc_on && xg + v >= d.lo[0] && xg + v < d.hi[0]) a += (double)ss * (double)ss;
-        }
+        for (int f = 0; f < 12; f++) c[f] = co[f].v[v];
+        float ss;
+        const float r = h.point(c, v, omega, &ss);
+        outv[v] = copy ? h.c[1 + v] : r;
+        if (acc_on && !copy && xg + v >= d.lo[0] && xg + v < d.hi[0])
+          a += (double)ss * (double)ss;
       }
       float *dst = pout + off;
       if (xvec) {
@@ -303,21 +367,12 @@ __device__ __forceinline__ bool ht_stage2_tile(const HtRings &R, RingPos &p2, Ri
           if (xg + v >= d.lo[0] && xg + v < d.hi[0]) dst[v] = outv[v];
       }
     }
-    ht_release(&R.ec[pc.slot], lane);
-    ring_next(pc, kHtSC);
-    ht_release(&R.e2[pm.slot], lane);
-    pm = pz;
-    pz = pp;
     off += sz;
   }
   // Coefficient plane zb+nzl (the first sweep's far halo plane).
   if (!ht_wait(&R.fc[pc.slot], pc.round & 1)) return false;
   ht_release(&R.ec[pc.slot], lane);
   ring_next(pc, kHtSC);
-  ht_release(&R.e2[pm.slot], lane);
-  ht_release(&R.e2[pz.slot], lane);
-  p2 = pz;
-  ring_next(p2, kHtS2);
   *acc += a;
   return true;
 }

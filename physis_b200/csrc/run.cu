@@ -431,16 +431,23 @@ static psb_status run_pipe(MapImpl **ms, const PipePlan &plan, int64_t *launches
 }
 
 // The same for a Himeno pair (two sweeps per launch, k_himeno_tb2.cu): each
-// launch runs m1's sweep then m2's, alternating A -> B and B -> A.
-static psb_status run_himeno_tb2(MapImpl **ms, int iter, int zchunk, int64_t *launches) {
+// launch runs m1's sweep then m2's, A -> the work grid S and S -> A in turn, with
+// A's rim in S. B keeps its own rim, which the second sweeps read, and is
+// written by the last iteration only (single sweeps, from S where S holds the
+// state), so both grids end as after single sweeps whatever rims they came with.
+static psb_status run_himeno_tb2(MapImpl **ms, GridImpl *S, int iter, int zchunk,
+                                 int64_t *launches) {
   Runtime &r = rt();
-  GridImpl *A = ms[0]->grids[0], *B = ms[0]->grids[1];
-  const int F = (iter - 1) & ~1;
-  for (int f = 0; f < F; f++)
-    PSB_CHECK(himeno_tb2_launch(*ms[0], *ms[1], f & 1 ? B : A, f & 1 ? A : B, zchunk, r.stream,
-                                launches));
-  for (int it = F; it < iter; it++) PSB_CHECK(launch_iteration(ms, 2, launches));
-  return PSB_OK;
+  GridImpl *A = ms[0]->grids[0], *g[2] = {A, S};
+  PSB_CHECK(himeno_rim_copy(*ms[0], S, r.stream, launches));
+  for (int f = 0; f < iter - 1; f++)
+    PSB_CHECK(himeno_tb2_launch(*ms[0], *ms[1], g[f & 1], g[(f & 1) ^ 1], zchunk, true,
+                                r.stream, launches));
+  ms[0]->grids[0] = g[(iter - 1) & 1];
+  const psb_status st = launch_map(*ms[0], -1, launches);
+  ms[0]->grids[0] = A;
+  PSB_CHECK(st);
+  return launch_map(*ms[1], -1, launches);
 }
 
 static psb_status run_maps(MapImpl **ms, int n, int iter) {
@@ -467,16 +474,17 @@ static psb_status run_maps(MapImpl **ms, int n, int iter) {
   if (r.impl != PSB_IMPL_PLAIN && r.impl != PSB_IMPL_GENERIC && himeno_tb2_pair(ms, n) &&
       iter >= 3) {
     // Without an entry two sweeps per pass: faster than single sweeps on
-    // every shape timed (65x65x129 9.6 against 11.9 us a sweep, 200^3 94
-    // against 142, 35x40x50 7.3 against 9.1).
+    // every shape timed (65x65x129 7.9 against 11.9 us a sweep, 200^3 58
+    // against 142).
     psb_tune_config cfg;
     const int *dims = ms[0]->grids[0]->pub.dim;
     if (!tune_find(PSB_KERNEL_HIMENO19, PS_FLOAT, dims, &cfg)) {
       cfg.t_depth = 2;
       cfg.z_chunk = himeno_tb2_chunk(ms[0]->dom);
     }
-    if (cfg.t_depth == 2) {
-      PSB_CHECK(run_himeno_tb2(ms, iter, cfg.z_chunk, &launches));
+    GridImpl *S = cfg.t_depth == 2 ? grid_work(ms[0]->grids[0]) : nullptr;
+    if (S) {
+      PSB_CHECK(run_himeno_tb2(ms, S, iter, cfg.z_chunk, &launches));
       PSB_TRY(cudaEventRecord(r.ev_stop, r.stream));
       legacy_join_out();
       r.last_launches = launches;

@@ -218,6 +218,49 @@ static void grid_attach(GridImpl *g) {
   set_dev_struct(g, g->pub.p0);
 }
 
+// The runtime's work grid: one allocation, as large as the largest grid that
+// asked for it (a new state of a known shape finds it there). Its users run
+// under the runtime's lock on its stream. Given back with the last grid, when a
+// grid allocation fails, and at the end.
+static GridImpl *g_work = nullptr;
+static size_t g_work_bytes = 0;
+static int64_t g_grids = 0;  // live allocations of grid_alloc
+
+static void work_release() {
+  if (!g_work) return;
+  cudaStreamSynchronize(rt().stream);
+  cudaFree(g_work->alloc);
+  delete g_work;
+  g_work = nullptr;
+  g_work_bytes = 0;
+}
+
+GridImpl *grid_work(const GridImpl *g) {
+  std::lock_guard<std::recursive_mutex> lk(rt().mu);
+  if (g_work && g_work->type == g->type && g_work->layout == g->layout &&
+      g_work->pub.num_dims == g->pub.num_dims &&
+      memcmp(g_work->pub.dim, g->pub.dim, sizeof(g->pub.dim)) == 0)
+    return g_work;
+  if (g_work && g_work_bytes < g->alloc_bytes) work_release();
+  void *mem = g_work ? g_work->alloc : nullptr;
+  if (!mem) {
+    // Not where it would take more than half of what the user's next grids have.
+    size_t free_bytes = 0, total = 0;
+    if (cudaMemGetInfo(&free_bytes, &total) != cudaSuccess || g->alloc_bytes > free_bytes / 2 ||
+        cudaMalloc(&mem, g->alloc_bytes) != cudaSuccess) {
+      cudaGetLastError();
+      return nullptr;
+    }
+    g_work_bytes = g->alloc_bytes;
+  }
+  delete g_work;
+  g_work = grid_describe(g->type, g->pub.elm_size, g->pub.num_dims, g->pub.dim, g->layout);
+  g_work->alloc = mem;
+  grid_attach(g_work);
+  g_work->ghost_valid = PSB_BOUNDARY_NONE;
+  return g_work;
+}
+
 static psb_status grid_alloc(int type, int elm_size, int nd, const int *dims, int layout,
                              GridImpl **out) {
   *out = nullptr;
@@ -228,6 +271,12 @@ static psb_status grid_alloc(int type, int elm_size, int nd, const int *dims, in
   PSB_CHECK(ensure_init());
   GridImpl *g = grid_describe(type, elm_size, nd, dims, layout);
   cudaError_t e = cudaMalloc(&g->alloc, g->alloc_bytes);
+  std::lock_guard<std::recursive_mutex> lk(rt().mu);
+  if (e == cudaErrorMemoryAllocation && g_work) {
+    cudaGetLastError();
+    work_release();
+    e = cudaMalloc(&g->alloc, g->alloc_bytes);
+  }
   if (e != cudaSuccess) {
     delete g;
     cudaGetLastError();
@@ -241,6 +290,7 @@ static psb_status grid_alloc(int type, int elm_size, int nd, const int *dims, in
     return cuda_status(e, "cudaMemset(grid)");
   }
   grid_attach(g);
+  g_grids++;
   *out = g;
   return PSB_OK;
 }
@@ -303,6 +353,8 @@ static void grid_free(GridImpl *g) {
   } else if (g->alloc) {
     cudaStreamSynchronize(rt().stream);
     PSB_FATAL(cudaFree(g->alloc));
+    std::lock_guard<std::recursive_mutex> lk(rt().mu);
+    if (--g_grids == 0) work_release();
   }
   g->magic = 0;
   delete g;
@@ -466,6 +518,7 @@ void PSFinalize(void) {
   Runtime &r = rt();
   if (!r.inited) return;
   cudaStreamSynchronize(r.stream);
+  work_release();
   for (auto &kv : r.graphs) cudaGraphExecDestroy(kv.second);
   r.graphs.clear();
   for (auto &m : r.maps) {

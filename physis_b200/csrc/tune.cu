@@ -231,7 +231,7 @@ static double time_config(MapImpl &m, const psb_tune_config &cfg, int reps) {
       psb_status st;
       if (m.kernel_id == PSB_KERNEL_HIMENO19)
         st = cfg.t_depth == 2 ? himeno_tb2_launch(m, m, m.grids[0], m.grids[1], cfg.z_chunk,
-                                                  r.stream, &launches)
+                                                  false, r.stream, &launches)
                               : himeno_launch(m, cfg, r.stream, &launches);
       else
         st = cfg.t_depth == 2
@@ -374,7 +374,7 @@ psb_status psb_autotune(int kernel_id, int type, const PSIndex *dims, int force,
       c.t_depth = 2;
       cands.push_back(c);
     }
-  // Himeno, two sweeps per pass (64 x 8 tiles; the single-sweep fields of
+  // Himeno, two sweeps per pass (64 x 12 tiles; the single-sweep fields of
   // the entry are the default shape, used for maps run alone).
   if (kernel_id == PSB_KERNEL_HIMENO19)
     for (int zc : {16, 32, 64}) {

@@ -22,3 +22,32 @@ def test_run_without_an_entry_equals_plain(shape, sweeps):
     want, wgosa = U.himeno_gpu(p, coef, 0.8, sweeps, impl=ps.IMPL_PLAIN)
     assert U.bits_equal(got, want)
     assert np.allclose(gosa, wgosa, rtol=1e-12, atol=0)
+
+
+# The second grid comes with values of its own (its rim stays in every second
+# sweep), the domain is the interior or a part of it, and the passes end in the
+# first grid (odd pairs) or in the work grid (even ones).
+@pytest.mark.parametrize("shape,cut", [((9, 11, 67), 0), ((20, 70, 131), 0), ((30, 41, 140), 3)])
+@pytest.mark.parametrize("pairs", [3, 4, 5])
+def test_grids_with_different_rims_equal_plain(shape, cut, pairs):
+    ps.PSInit()
+    p, coef = U.himeno_inputs(shape, 12)
+    other = np.random.default_rng(5).random(shape, dtype=np.float32)
+    nz, ny, nx = shape
+    out = []
+    for impl in (ps.IMPL_AUTO, ps.IMPL_PLAIN):
+        gs = [ps.grid_new(ps.PS_FLOAT, (nx, ny, nz)) for _ in range(14)]
+        for g, a in zip(gs, [p, other] + list(coef)):
+            ps.PSGridCopyin(g, a)
+        d = ps.PSDomain3DNew(1 + cut, nx - 1 - cut, 1, ny - 1 - cut, 1 + cut, nz - 1)
+        ps.set_impl(impl)
+        try:
+            m1 = ps.PSStencilMap(ps.HIMENO19, d, *gs, 0.8)
+            m2 = ps.PSStencilMap(ps.HIMENO19, d, gs[1], gs[0], *gs[2:], 0.8)
+            ps.PSStencilRun(m1, m2, pairs)
+            out.append([ps.PSGridCopyout(g) for g in gs[:2]])
+        finally:
+            ps.set_impl(ps.IMPL_AUTO)
+            for g in gs:
+                ps.PSGridFree(g)
+    assert U.bits_equal(out[0][0], out[1][0]) and U.bits_equal(out[0][1], out[1][1])
