@@ -206,7 +206,7 @@ int himeno_tb2_chunk(const __PSDomain &dom);  // z chunk of the pass over a doma
 // output grid's on the way (Runtime::rim_run).
 psb_status himeno_rim_copy(const MapImpl &m, GridImpl *dst, cudaStream_t s, int64_t *launches);
 psb_status himeno_tb2_launch(MapImpl &m1, MapImpl &m2, GridImpl *in, GridImpl *out,
-                             int zchunk, bool rims, cudaStream_t s, int64_t *launches);
+                             int zchunk, bool rims, bool last, cudaStream_t s, int64_t *launches);
 psb_status generic_tma_launch(MapImpl &m, const GenericDesc &gd, int color, cudaStream_t s,
                               int64_t *launches);
 void generic_note_impl(int impl);

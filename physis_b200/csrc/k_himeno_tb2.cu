@@ -21,9 +21,9 @@
 // values outside the domain are those of the grid the first sweep writes (it
 // leaves them there), so the result equals two single sweeps bit for bit, also
 // where the two grids' rims differ: a run keeps that grid untouched until its
-// last two sweeps and alternates between the input and the work grid, whose
-// rim is the input's (himeno_rim_copy, which also finds out whether the rims
-// differ at all). The residual
+// last pass, which stores its first sweep there, and alternates between the
+// input and the work grid, whose rim is the input's (himeno_rim_copy, which
+// also finds out whether the rims differ at all). The residual
 // sum of ss*ss of each sweep is accumulated over the tile's own points in
 // FP64 and combined per sweep in a fixed order (one partial per CTA, the
 // last CTA adds them in index order) into the history of the map whose
@@ -124,7 +124,7 @@ __global__ void __launch_bounds__(kHtThreads, 1)
       bad = rim ? !ht_stage1_tile<true>(R, p1, pc, p2, tid - 32, lane, d, omega, x0, y0, zb, nzl,
                                         true, &acc, hg.rim)
                 : !ht_stage1_tile<false>(R, p1, pc, p2, tid - 32, lane, d, omega, x0, y0, zb, nzl,
-                                         true, &acc);
+                                         true, &acc, hg.rim);
     }
   } else {
     RingPos p2{0, 0}, pc{0, 0};
@@ -304,9 +304,9 @@ psb_status himeno_rim_copy(const MapImpl &m, GridImpl *dst, cudaStream_t s, int6
 // residuals go to their histories when both maps have them enabled). in holds
 // the rim of m1's input grid; the rim of m1's output grid is read, not written.
 // rims: himeno_rim_copy ran for these maps (else both grids' rims are taken to
-// be the same).
+// be the same). last: the first sweep is stored in m1's output grid.
 psb_status himeno_tb2_launch(MapImpl &m1, MapImpl &m2, GridImpl *in, GridImpl *out,
-                             int zchunk, bool rims, cudaStream_t s, int64_t *launches) {
+                             int zchunk, bool rims, bool last, cudaStream_t s, int64_t *launches) {
   Runtime &r = rt();
   const CUtensorMap *pmap = nullptr;
   PSB_CHECK(get_tmap(in, kHtBX, kHtBY1, &pmap));
@@ -329,7 +329,8 @@ psb_status himeno_tb2_launch(MapImpl &m1, MapImpl &m2, GridImpl *in, GridImpl *o
   }
   HtGeom hg;
   const GridImpl *B = m1.grids[1];
-  hg.rim = HtRim{(const float *)B->view().origin, B->sy, B->sz, B->pub.dim[0], B->pub.dim[1]};
+  hg.rim = HtRim{(const float *)B->view().origin, B->sy, B->sz, B->pub.dim[0], B->pub.dim[1],
+                 last ? (float *)B->view().origin : nullptr};
   hg.rim_differs = r.d_error + 2;
   hg.rim_run = rims ? r.rim_run : -1;
   hg.ax0 = in->pad_left;

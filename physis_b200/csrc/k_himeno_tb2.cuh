@@ -171,13 +171,15 @@ __device__ __forceinline__ bool ht_begin(HimenoWalk<V> &h, RingPos &p, int S, ui
   return true;
 }
 
-// Where first-sweep values outside the domain come from: the grid that the
-// first sweep writes, as a sweep leaves them there (p: logical (0,0,0); nx, ny:
-// points inside it).
+// The grid that the first sweep writes. Its values outside the domain are the
+// first sweep's there, as a sweep leaves them (p: logical (0,0,0); nx, ny:
+// points inside the grid). mid: p where the first sweep's own values are to be
+// stored too (a run's last pass), else null.
 struct HtRim {
   const float *p;
   int64_t sy, sz;
   int nx, ny;
+  float *mid;
 };
 
 // Stage-1 warps (thread t in [0, 224)): the first sweep of one tile into R2.
@@ -245,6 +247,16 @@ __device__ __forceinline__ bool ht_stage1_tile(const HtRings &R, RingPos &p1, Ri
 #pragma unroll
       for (int v = 0; v < kHtV; v++)
         if (!(z_in && row_in && xg + v >= d.lo[0] && xg + v < d.hi[0])) outv[v] = w[v];
+    }
+    if (rim.mid && z_own && row_own) {
+      float *q = rim.mid + xg + (int64_t)yg * rim.sy + (int64_t)z * rim.sz;
+      if (xy_in) {
+        *reinterpret_cast<float4 *>(q) = make_float4(outv[0], outv[1], outv[2], outv[3]);
+      } else {
+#pragma unroll
+        for (int v = 0; v < kHtV; v++)
+          if (xg + v >= d.lo[0] && xg + v < d.hi[0]) q[v] = outv[v];
+      }
     }
     // The first-sweep plane z into the next stage of R2.
     if (p2.round > 0 && !ht_wait(&R.e2[p2.slot], (p2.round - 1) & 1)) return false;

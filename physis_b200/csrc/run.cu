@@ -432,22 +432,26 @@ static psb_status run_pipe(MapImpl **ms, const PipePlan &plan, int64_t *launches
 
 // The same for a Himeno pair (two sweeps per launch, k_himeno_tb2.cu): each
 // launch runs m1's sweep then m2's, A -> the work grid S and S -> A in turn, with
-// A's rim in S. B keeps its own rim, which the second sweeps read, and is
-// written by the last iteration only (single sweeps, from S where S holds the
-// state), so both grids end as after single sweeps whatever rims they came with.
+// A's rim in S, so that the last one is S -> A; an odd number starts from a copy
+// of A. B keeps its own rim, which the second sweeps read, and is written by the
+// last launch's first sweep only, so both grids end as after single sweeps
+// whatever rims they came with.
 static psb_status run_himeno_tb2(MapImpl **ms, GridImpl *S, int iter, int zchunk,
                                  int64_t *launches) {
   Runtime &r = rt();
-  GridImpl *A = ms[0]->grids[0], *g[2] = {A, S};
+  GridImpl *A = ms[0]->grids[0], *in = A, *out = S;
+  if (iter & 1) {
+    PSB_TRY(cudaMemcpyAsync(S->alloc, A->alloc, A->alloc_bytes, cudaMemcpyDeviceToDevice,
+                            r.stream));
+    std::swap(in, out);
+  }
   PSB_CHECK(himeno_rim_copy(*ms[0], S, r.stream, launches));
-  for (int f = 0; f < iter - 1; f++)
-    PSB_CHECK(himeno_tb2_launch(*ms[0], *ms[1], g[f & 1], g[(f & 1) ^ 1], zchunk, true,
-                                r.stream, launches));
-  ms[0]->grids[0] = g[(iter - 1) & 1];
-  const psb_status st = launch_map(*ms[0], -1, launches);
-  ms[0]->grids[0] = A;
-  PSB_CHECK(st);
-  return launch_map(*ms[1], -1, launches);
+  for (int i = 0; i < iter; i++) {
+    PSB_CHECK(himeno_tb2_launch(*ms[0], *ms[1], in, out, zchunk, true, i == iter - 1, r.stream,
+                                launches));
+    std::swap(in, out);
+  }
+  return PSB_OK;
 }
 
 static psb_status run_maps(MapImpl **ms, int n, int iter) {
@@ -472,7 +476,7 @@ static psb_status run_maps(MapImpl **ms, int n, int iter) {
   // Single steps read the halos prepared here.
   for (int i = 0; i < n && pipe; i++) PSB_CHECK(prepare_ghosts(*ms[i]));
   if (r.impl != PSB_IMPL_PLAIN && r.impl != PSB_IMPL_GENERIC && himeno_tb2_pair(ms, n) &&
-      iter >= 3) {
+      iter >= 2) {
     // Without an entry two sweeps per pass: faster than single sweeps on
     // every shape timed (65x65x129 7.9 against 11.9 us a sweep, 200^3 58
     // against 142).

@@ -231,7 +231,7 @@ static double time_config(MapImpl &m, const psb_tune_config &cfg, int reps) {
       psb_status st;
       if (m.kernel_id == PSB_KERNEL_HIMENO19)
         st = cfg.t_depth == 2 ? himeno_tb2_launch(m, m, m.grids[0], m.grids[1], cfg.z_chunk,
-                                                  false, r.stream, &launches)
+                                                  false, false, r.stream, &launches)
                               : himeno_launch(m, cfg, r.stream, &launches);
       else
         st = cfg.t_depth == 2

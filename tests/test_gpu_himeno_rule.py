@@ -25,10 +25,10 @@ def test_run_without_an_entry_equals_plain(shape, sweeps):
 
 
 # The second grid comes with values of its own (its rim stays in every second
-# sweep), the domain is the interior or a part of it, and the passes end in the
-# first grid (odd pairs) or in the work grid (even ones).
+# sweep), the domain is the interior or a part of it, and the passes start from
+# the first grid (even pairs) or from a copy of it (odd ones).
 @pytest.mark.parametrize("shape,cut", [((9, 11, 67), 0), ((20, 70, 131), 0), ((30, 41, 140), 3)])
-@pytest.mark.parametrize("pairs", [3, 4, 5])
+@pytest.mark.parametrize("pairs", [2, 3, 4, 5])
 def test_grids_with_different_rims_equal_plain(shape, cut, pairs):
     ps.PSInit()
     p, coef = U.himeno_inputs(shape, 12)
