@@ -17,6 +17,8 @@ struct GpArgs {
   int color;
   int tx_shift;          // log2 of the threads along x
   int tiles_x, tiles_y;  // blocks along x and y
+  unsigned mul_x, mul_y; // b / tiles_x = (b * mul_x) >> shift_x for a block index b
+  int shift_x, shift_y;
 };
 
 // Indices of the periodic form (i + n) % n: within one period of the grid
@@ -48,10 +50,11 @@ struct GpAt {
 
 template <int ND, int U, bool COLORED>
 __device__ __forceinline__ GpAt gp_position(const GpArgs &q) {
-  int b = blockIdx.x;
-  const int bx = b % q.tiles_x;
-  b /= q.tiles_x;
-  const int by = b % q.tiles_y, bz = b / q.tiles_y;
+  const unsigned b = blockIdx.x;
+  const unsigned row = ND == 1 ? 0 : (unsigned)(((uint64_t)b * q.mul_x) >> q.shift_x);
+  const int bx = (int)(b - row * q.tiles_x);
+  const int bz = ND < 3 ? 0 : (int)(((uint64_t)row * q.mul_y) >> q.shift_y);
+  const int by = (int)row - bz * q.tiles_y;
   const int tx = threadIdx.x & ((1 << q.tx_shift) - 1), ty = threadIdx.x >> q.tx_shift;
   const int xi = (bx << q.tx_shift) + tx, yi = by * (kGpThreads >> q.tx_shift) + ty;
   GpAt at;
