@@ -451,6 +451,7 @@ static psb_status run_himeno_tb2(MapImpl **ms, GridImpl *S, int iter, int zchunk
                                 launches));
     std::swap(in, out);
   }
+  A->ghost_valid = ms[0]->grids[1]->ghost_valid = PSB_BOUNDARY_NONE;
   return PSB_OK;
 }
 

@@ -51,3 +51,34 @@ def test_grids_with_different_rims_equal_plain(shape, cut, pairs):
             for g in gs:
                 ps.PSGridFree(g)
     assert U.bits_equal(out[0][0], out[1][0]) and U.bits_equal(out[0][1], out[1][1])
+
+
+def test_halos_are_refreshed_after_a_run():
+    """Both grids' halos (filled for periodic reads before the run) are stale
+    after it: a periodic read two cells away sees the new values."""
+    ps.PSInit()
+    shape = (12, 14, 66)
+    nz, ny, nx = shape
+    p, coef = U.himeno_inputs(shape, 13)
+    st = ps.GenericStencil(3, [(ps.PS_FLOAT, (0, 1, 2))] * 2, 1, ps.PS_FLOAT,
+                           [(ps.get(0, [-2, 0, 0], ps.BOUNDARY_PERIODIC), ps.const(1.0)),
+                            (ps.get(0, [0, 2, 0], ps.BOUNDARY_PERIODIC), ps.const(1.0))])
+    gs = [ps.grid_new(ps.PS_FLOAT, (nx, ny, nz)) for _ in range(15)]
+    try:
+        for g, a in zip(gs, [p, p] + list(coef)):
+            ps.PSGridCopyin(g, a)
+        whole = ps.PSDomain3DNew(0, nx, 0, ny, 0, nz)
+        reads = [ps.PSStencilMap(st.kernel_id, whole, g, gs[14]) for g in gs[:2]]
+        for m in reads:
+            ps.PSStencilRun(m, 1)
+        d = ps.PSDomain3DNew(1, nx - 1, 1, ny - 1, 1, nz - 1)
+        ps.PSStencilRun(ps.PSStencilMap(ps.HIMENO19, d, *gs[:14], 0.8),
+                        ps.PSStencilMap(ps.HIMENO19, d, gs[1], gs[0], *gs[2:14], 0.8), 4)
+        for g, m in zip(gs[:2], reads):
+            a = ps.PSGridCopyout(g)
+            ps.PSStencilRun(m, 1)
+            want = np.roll(a, 2, axis=2) + np.roll(a, -2, axis=1)
+            assert U.bits_equal(ps.PSGridCopyout(gs[14]), want)
+    finally:
+        for g in gs:
+            ps.PSGridFree(g)
