@@ -169,7 +169,7 @@ static std::string gt_jit_source(const GtTable &tab, bool dbl, bool fma, std::st
 // The plane-by-plane form (gt_body_planes) needs a packed table whose terms
 // come in plane order over two or three planes, and pays from eight terms on.
 // Float at 512^3, this form against the window form: 27 equal coefficients
-// 239 us against 464 (FMA mode 235 against 400), 27 distinct ones 328 against
+// 232 us against 464 (FMA mode 233 against 400), 27 distinct ones 328 against
 // 464; a 7-term star 212 against 205; a 13-term star over five planes, whose
 // running sums leave too few registers, 272 against 243.
 static bool gt_plane_form(const GtTable &tab, const GtGeom &geo) {
