@@ -191,7 +191,8 @@ __global__ void __launch_bounds__(kHtThreads, 1)
 
 // Both maps of PSStencilRun(m1(p0 -> p1), m2(p1 -> p0), n) form a Himeno
 // pair the two-sweep pass can advance: pitched float grids of one shape and
-// layout, the same coefficient grids, domain and omega.
+// layout, the same coefficient grids (none of them a pressure grid), domain
+// and omega.
 bool himeno_tb2_pair(MapImpl **ms, int n) {
   if (n != 2) return false;
   const MapImpl &a = *ms[0], &b = *ms[1];
@@ -200,8 +201,11 @@ bool himeno_tb2_pair(MapImpl **ms, int n) {
   if (b.grids[0] != a.grids[1] || b.grids[1] != a.grids[0] || a.grids[0] == a.grids[1])
     return false;
   if (memcmp(&a.dom, &b.dom, sizeof(a.dom)) != 0) return false;
+  // A coefficient that is one of the two pressure grids changes from sweep to
+  // sweep; single sweeps read it at the point itself, before its store.
   for (int i = 2; i < 14; i++)
-    if (a.grids[i] != b.grids[i]) return false;
+    if (a.grids[i] != b.grids[i] || a.grids[i] == a.grids[0] || a.grids[i] == a.grids[1])
+      return false;
   const GridImpl *g0 = a.grids[0];
   for (int i = 0; i < 14; i++) {
     const GridImpl *g = a.grids[i];

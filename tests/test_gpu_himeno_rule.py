@@ -82,3 +82,36 @@ def test_halos_are_refreshed_after_a_run():
     finally:
         for g in gs:
             ps.PSGridFree(g)
+
+
+# Slots of the coefficient (wrk1, bnd, the first field) that is one of the two
+# pressure grids: it changes with every sweep, and each point reads its own
+# before it is stored.
+@pytest.mark.parametrize("slot", [12, 13, 2])
+@pytest.mark.parametrize("pressure", [0, 1])
+def test_coefficient_that_is_a_pressure_grid_equals_plain(slot, pressure):
+    ps.PSInit()
+    shape, pairs = (20, 30, 131), 4
+    nz, ny, nx = shape
+    p, coef = U.himeno_inputs(shape, 14)
+    other = np.random.default_rng(6).random(shape, dtype=np.float32)
+    out = []
+    for impl in (ps.IMPL_AUTO, ps.IMPL_PLAIN):
+        gs = [ps.grid_new(ps.PS_FLOAT, (nx, ny, nz)) for _ in range(14)]
+        for g, a in zip(gs, [p, other] + list(coef)):
+            ps.PSGridCopyin(g, a)
+        bound = list(gs)
+        bound[slot] = gs[pressure]
+        d = ps.PSDomain3DNew(1, nx - 1, 1, ny - 1, 1, nz - 1)
+        ps.set_impl(impl)
+        try:
+            m1 = ps.PSStencilMap(ps.HIMENO19, d, *bound, 0.8)
+            m2 = ps.PSStencilMap(ps.HIMENO19, d, bound[1], bound[0], *bound[2:], 0.8)
+            ps.PSStencilRun(m1, m2, pairs)
+            assert ps.last_run_stats()[1] == 2 * pairs  # single sweeps
+            out.append([ps.PSGridCopyout(g) for g in gs[:2]])
+        finally:
+            ps.set_impl(ps.IMPL_AUTO)
+            for g in gs:
+                ps.PSGridFree(g)
+    assert U.bits_equal(out[0][0], out[1][0]) and U.bits_equal(out[0][1], out[1][1])
