@@ -30,64 +30,16 @@
 
 namespace psb {
 
-// Elements of a segment per thread: loads in flight (1 KB a warp).
-template <typename T>
-constexpr int kReduceU = 32 / (int)sizeof(T);
-constexpr int kReduceAcc = 4;  // accumulators per thread
-
 template <typename T, int OP>
 __global__ void __launch_bounds__(256) k_reduce(GridView g, Dom3 d, ReduceScratch sc) {
   __shared__ RAcc scratch[32];
   __shared__ int is_last;
-  constexpr int U = kReduceU<T>;
-  const int lane = threadIdx.x & 31;
   const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
   const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
-  const int rx = d.hi[0] - d.lo[0], ry = d.hi[1] - d.lo[1], rz = d.hi[2] - d.lo[2];
-  const int segs = (int)(((int64_t)rx + 32 * U - 1) / (32 * U));
-  // This warp's segments, `nwarps` apart in (z, y, segment) order, advanced
-  // by carries (64-bit: a row may be up to 2^31-1 elements long).
-  const int64_t drow = nwarps / segs, row0 = warp / segs;
-  const int ds = (int)(nwarps % segs), dy = (int)(drow % ry);
-  const int64_t dz = drow / ry;
-  int s = (int)(warp % segs), y = (int)(row0 % ry);
-  int64_t z = row0 / ry;
   const T *base = (const T *)g.origin + d.lo[0] + (int64_t)d.lo[1] * g.sy + (int64_t)d.lo[2] * g.sz;
-  RAcc a[kReduceAcc];
-#pragma unroll
-  for (int u = 0; u < U; u++) a[u] = racc_init(OP);
-  while (z < rz) {
-    const T *row = base + y * g.sy + z * g.sz;
-    const int64_t x0 = (int64_t)s * (32 * U) + lane;
-    T v[U];
-    if (x0 - lane + 32 * U <= rx) {
-#pragma unroll
-      for (int u = 0; u < U; u++) v[u] = row[x0 + 32 * u];
-#pragma unroll
-      for (int u = 0; u < U; u++) racc_add(OP, a[u % kReduceAcc], (double)v[u]);
-    } else {
-#pragma unroll
-      for (int u = 0; u < U; u++)
-        if (x0 + 32 * u < rx) racc_add(OP, a[u % kReduceAcc], (double)row[x0 + 32 * u]);
-    }
-    s += ds;
-    int cy = 0;
-    if (s >= segs) {
-      s -= segs;
-      cy = 1;
-    }
-    // y + dy + cy may exceed 2^31 - 1 before the carry.
-    int64_t y2 = (int64_t)y + dy + cy;
-    z += dz;
-    if (y2 >= ry) {
-      y2 -= ry;
-      z++;
-    }
-    y = (int)y2;
-  }
-#pragma unroll
-  for (int u = 1; u < kReduceAcc; u++) a[0] = racc_merge(OP, a[0], a[u]);
-  RAcc b = racc_block(OP, a[0], scratch);
+  const RAcc a = reduce_thread<T, OP>(base, g.sy, g.sz, d.hi[0] - d.lo[0], d.hi[1] - d.lo[1],
+                                      d.hi[2] - d.lo[2], warp, nwarps, threadIdx.x & 31);
+  RAcc b = racc_block(OP, a, scratch);
   if (threadIdx.x == 0) {
     sc.partials[blockIdx.x] = b;
     __threadfence();
