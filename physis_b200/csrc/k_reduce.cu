@@ -118,10 +118,9 @@ psb_status reduce_view(const GridView &v, int type, int op, const Dom3 &dom, dou
   static std::mutex mu;
   std::lock_guard<std::mutex> lk(mu);
   static double *host = nullptr, *mapped = nullptr;
-  if (!host) {
+  if (!host)
     PSB_TRY(cudaHostAlloc(&host, sizeof(double), cudaHostAllocMapped | cudaHostAllocPortable));
-    PSB_TRY(cudaHostGetDevicePointer(&mapped, host, 0));
-  }
+  if (!mapped) PSB_TRY(cudaHostGetDevicePointer(&mapped, host, 0));
   sc.result = mapped;
   if (!reduce_launch_typed(type, v, dom, op, sc, s)) return set_status(PSB_ERR_INVALID);
   PSB_TRY(cudaGetLastError());
