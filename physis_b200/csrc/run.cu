@@ -455,6 +455,23 @@ static psb_status run_himeno_tb2(MapImpl **ms, GridImpl *S, int iter, int zchunk
   return PSB_OK;
 }
 
+// The end of a run, whichever way it took: its time, its launches, the trace
+// line.
+static psb_status finish_run(int64_t launches) {
+  Runtime &r = rt();
+  PSB_TRY(cudaEventRecord(r.ev_stop, r.stream));
+  legacy_join_out();
+  r.last_launches = launches;
+  r.last_timed = true;
+  if (__ps_trace) {
+    float ms_ = 0;
+    cudaEventSynchronize(r.ev_stop);
+    cudaEventElapsedTime(&ms_, r.ev_start, r.ev_stop);
+    fprintf(__ps_trace, "Physis: Stencil finished (time: %f)\n", ms_);
+  }
+  return PSB_OK;
+}
+
 static psb_status run_maps(MapImpl **ms, int n, int iter) {
   Runtime &r = rt();
   if (iter <= 0) return PSB_OK;
@@ -468,11 +485,7 @@ static psb_status run_maps(MapImpl **ms, int n, int iter) {
   PipePlan plan;
   if (pipe && pipe_plan(ms, iter, &plan)) {
     PSB_CHECK(run_pipe(ms, plan, &launches));
-    PSB_TRY(cudaEventRecord(r.ev_stop, r.stream));
-    legacy_join_out();
-    r.last_launches = launches;
-    r.last_timed = true;
-    return PSB_OK;
+    return finish_run(launches);
   }
   // Single steps read the halos prepared here.
   for (int i = 0; i < n && pipe; i++) PSB_CHECK(prepare_ghosts(*ms[i]));
@@ -490,11 +503,7 @@ static psb_status run_maps(MapImpl **ms, int n, int iter) {
     GridImpl *S = cfg.t_depth == 2 ? grid_work(ms[0]->grids[0]) : nullptr;
     if (S) {
       PSB_CHECK(run_himeno_tb2(ms, S, iter, cfg.z_chunk, &launches));
-      PSB_TRY(cudaEventRecord(r.ev_stop, r.stream));
-      legacy_join_out();
-      r.last_launches = launches;
-      r.last_timed = true;
-      return PSB_OK;
+      return finish_run(launches);
     }
   }
   // The first iteration always runs eagerly: it performs every lazy set-up
@@ -544,17 +553,7 @@ static psb_status run_maps(MapImpl **ms, int n, int iter) {
     }
     for (int k = 0; k < rest % unroll; k++) PSB_CHECK(launch_iteration(ms, n, &launches));
   }
-  PSB_TRY(cudaEventRecord(r.ev_stop, r.stream));
-  legacy_join_out();
-  r.last_launches = launches;
-  r.last_timed = true;
-  if (__ps_trace) {
-    float ms_ = 0;
-    cudaEventSynchronize(r.ev_stop);
-    cudaEventElapsedTime(&ms_, r.ev_start, r.ev_stop);
-    fprintf(__ps_trace, "Physis: Stencil finished (time: %f)\n", ms_);
-  }
-  return PSB_OK;
+  return finish_run(launches);
 }
 
 static psb_status make_map(int kernel_id, const __PSDomain *dom, __PSGrid *const *grids,
