@@ -856,7 +856,7 @@ static psb_status dev_reserve(T **p, size_t *cap, size_t bytes) {
   cudaFree(*p);
   *p = nullptr;
   *cap = 0;
-  PSB_TRY(cudaMalloc((void **)p, want));
+  PSB_TRY(device_malloc(p, want));
   *cap = want;
   return PSB_OK;
 }
@@ -1265,7 +1265,7 @@ psb_status batch_prepare(psb_batch *b, const std::vector<int> &steps, const std:
                           sizeof(int64_t) * (G.max_steps + 1)));
     PSB_TRY(cudaMemcpy(G.d_step_offset, G.step_offset.data(), sizeof(int64_t) * (G.max_steps + 1),
                        cudaMemcpyHostToDevice));
-    if (!G.d_cursor) PSB_TRY(cudaMalloc(&G.d_cursor, sizeof(unsigned long long)));
+    if (!G.d_cursor) PSB_TRY(device_malloc(&G.d_cursor, sizeof(unsigned long long)));
     int per_sm = 0;
     if (gi == 0) {
       PSB_TRY(cudaFuncSetAttribute(k_batch<0>, cudaFuncAttributePreferredSharedMemoryCarveout,

@@ -169,8 +169,22 @@ psb_status launch_halo_fill(GridImpl *g, int mode, cudaStream_t s);
 // zero fill on stream s, free after the work queued on s.
 size_t grid_pitched_bytes(int elm_size, const int *dims);
 // The runtime's work grid in g's shape and layout (contents unspecified), for use
-// on its stream under its lock; nullptr where the memory is short.
-GridImpl *grid_work(const GridImpl *g);
+// on its stream under its lock, while the object lives; null where the memory is
+// short.
+struct WorkGrid {
+  GridImpl *grid;
+  explicit WorkGrid(const GridImpl *g);
+  ~WorkGrid();
+  WorkGrid(const WorkGrid &) = delete;
+};
+// Every device allocation of the library: one that fails gets the work grid's
+// memory back and tries again.
+cudaError_t device_malloc(void **p, size_t bytes);
+cudaError_t device_malloc_async(void **p, size_t bytes, cudaMemPool_t pool, cudaStream_t s);
+template <typename T>
+cudaError_t device_malloc(T **p, size_t bytes) {
+  return device_malloc((void **)p, bytes);
+}
 psb_status grid_alloc_pool(int type, const int *dims, cudaMemPool_t pool, cudaStream_t s,
                            GridImpl **out);
 void grid_free_pool(GridImpl *g, cudaStream_t s);

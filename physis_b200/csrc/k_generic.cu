@@ -73,7 +73,7 @@ psb_status generic_upload(GenericDesc &d) {
     t.a[i] = compact(d.host.terms[i].a);
     t.b[i] = compact(d.host.terms[i].b);
   }
-  if (!d.dev) PSB_TRY(cudaMalloc(&d.dev, sizeof(GenTable)));
+  if (!d.dev) PSB_TRY(device_malloc(&d.dev, sizeof(GenTable)));
   PSB_TRY(cudaMemcpy(d.dev, &t, sizeof(t), cudaMemcpyHostToDevice));
   return PSB_OK;
 }

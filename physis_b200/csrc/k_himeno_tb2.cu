@@ -251,7 +251,7 @@ static psb_status ht_residual(MapImpl &m, int nblocks, Residual *r) {
   if (m.partials_cap < nblocks) {
     if (m.d_partials) cudaFree(m.d_partials);
     m.d_partials = nullptr;
-    PSB_TRY(cudaMalloc(&m.d_partials, sizeof(double) * nblocks));
+    PSB_TRY(device_malloc(&m.d_partials, sizeof(double) * nblocks));
     m.partials_cap = nblocks;
   }
   r->partials = m.d_partials;

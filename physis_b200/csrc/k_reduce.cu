@@ -98,7 +98,7 @@ psb_status reduce_scratch(ReduceScratch *sc) {
   static void *scratch = nullptr;
   if (!scratch) {
     size_t bytes = sizeof(RAcc) * kReduceMaxBlocks + 256;
-    PSB_TRY(cudaMalloc(&scratch, bytes));
+    PSB_TRY(device_malloc(&scratch, bytes));
     PSB_TRY(cudaMemset(scratch, 0, bytes));
   }
   sc->partials = (RAcc *)scratch;

@@ -500,10 +500,12 @@ static psb_status run_maps(MapImpl **ms, int n, int iter) {
       cfg.t_depth = 2;
       cfg.z_chunk = himeno_tb2_chunk(ms[0]->dom);
     }
-    GridImpl *S = cfg.t_depth == 2 ? grid_work(ms[0]->grids[0]) : nullptr;
-    if (S) {
-      PSB_CHECK(run_himeno_tb2(ms, S, iter, cfg.z_chunk, &launches));
-      return finish_run(launches);
+    if (cfg.t_depth == 2) {
+      const WorkGrid work(ms[0]->grids[0]);
+      if (work.grid) {
+        PSB_CHECK(run_himeno_tb2(ms, work.grid, iter, cfg.z_chunk, &launches));
+        return finish_run(launches);
+      }
     }
   }
   // The first iteration always runs eagerly: it performs every lazy set-up
@@ -906,13 +908,13 @@ psb_status psb_himeno_residual_enable(PSStencil h, int history_len) {
     return PSB_OK;
   }
   if (!m->d_ticket) {
-    PSB_TRY(cudaMalloc(&m->d_ticket, sizeof(unsigned) * 2));
+    PSB_TRY(device_malloc(&m->d_ticket, sizeof(unsigned) * 2));
     m->d_counter = m->d_ticket + 1;
   }
   PSB_TRY(cudaMemset(m->d_ticket, 0, sizeof(unsigned) * 2));
   if (m->d_history) cudaFree(m->d_history);
   m->d_history = nullptr;
-  PSB_TRY(cudaMalloc(&m->d_history, sizeof(double) * history_len));
+  PSB_TRY(device_malloc(&m->d_history, sizeof(double) * history_len));
   PSB_TRY(cudaMemset(m->d_history, 0, sizeof(double) * history_len));
   m->residual_len = history_len;
   return PSB_OK;

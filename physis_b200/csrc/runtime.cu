@@ -220,23 +220,47 @@ static void grid_attach(GridImpl *g) {
 
 // The runtime's work grid: one allocation, as large as the largest grid that
 // asked for it (a new state of a known shape finds it there). Its users run
-// under the runtime's lock on its stream. Given back with the last grid, when a
-// grid allocation fails, and at the end.
+// under the runtime's lock on its stream and hold WorkGrid while they queue
+// their launches. Given back with the last grid, when any device allocation of
+// the library fails, and at the end.
+static std::recursive_mutex g_work_mu;  // nothing that takes another lock runs under it
+static bool g_work_busy = false;        // between a WorkGrid's ends
 static GridImpl *g_work = nullptr;
 static size_t g_work_bytes = 0;
 static int64_t g_grids = 0;  // live allocations of grid_alloc
 
-static void work_release() {
-  if (!g_work) return;
+// False: there is none, or this thread is using it. (Another thread that does
+// is waited for; its launches are waited for here.)
+static bool work_release() {
+  std::lock_guard<std::recursive_mutex> lk(g_work_mu);
+  if (!g_work || g_work_busy) return false;
   cudaStreamSynchronize(rt().stream);
   cudaFree(g_work->alloc);
   delete g_work;
   g_work = nullptr;
   g_work_bytes = 0;
+  return true;
 }
 
-GridImpl *grid_work(const GridImpl *g) {
-  std::lock_guard<std::recursive_mutex> lk(rt().mu);
+cudaError_t device_malloc(void **p, size_t bytes) {
+  cudaError_t e = cudaMalloc(p, bytes);
+  if (e == cudaErrorMemoryAllocation && work_release()) {
+    cudaGetLastError();
+    e = cudaMalloc(p, bytes);
+  }
+  return e;
+}
+
+cudaError_t device_malloc_async(void **p, size_t bytes, cudaMemPool_t pool, cudaStream_t s) {
+  cudaError_t e = cudaMallocFromPoolAsync(p, bytes, pool, s);
+  if (e == cudaErrorMemoryAllocation && work_release()) {
+    cudaGetLastError();
+    e = cudaMallocFromPoolAsync(p, bytes, pool, s);
+  }
+  return e;
+}
+
+static GridImpl *work_acquire(const GridImpl *g) {
   if (g_work && g_work->type == g->type && g_work->layout == g->layout &&
       g_work->pub.num_dims == g->pub.num_dims &&
       memcmp(g_work->pub.dim, g->pub.dim, sizeof(g->pub.dim)) == 0)
@@ -244,9 +268,9 @@ GridImpl *grid_work(const GridImpl *g) {
   if (g_work && g_work_bytes < g->alloc_bytes) work_release();
   void *mem = g_work ? g_work->alloc : nullptr;
   if (!mem) {
-    // Not where it would take more than half of what the user's next grids have.
+    // Not where it would take more than an eighth of what is left for others.
     size_t free_bytes = 0, total = 0;
-    if (cudaMemGetInfo(&free_bytes, &total) != cudaSuccess || g->alloc_bytes > free_bytes / 2 ||
+    if (cudaMemGetInfo(&free_bytes, &total) != cudaSuccess || g->alloc_bytes > free_bytes / 8 ||
         cudaMalloc(&mem, g->alloc_bytes) != cudaSuccess) {
       cudaGetLastError();
       return nullptr;
@@ -261,6 +285,17 @@ GridImpl *grid_work(const GridImpl *g) {
   return g_work;
 }
 
+WorkGrid::WorkGrid(const GridImpl *g) {
+  g_work_mu.lock();
+  grid = work_acquire(g);
+  g_work_busy = true;
+}
+
+WorkGrid::~WorkGrid() {
+  g_work_busy = false;
+  g_work_mu.unlock();
+}
+
 static psb_status grid_alloc(int type, int elm_size, int nd, const int *dims, int layout,
                              GridImpl **out) {
   *out = nullptr;
@@ -270,13 +305,7 @@ static psb_status grid_alloc(int type, int elm_size, int nd, const int *dims, in
   if (elm_size <= 0) return set_status(PSB_ERR_INVALID);
   PSB_CHECK(ensure_init());
   GridImpl *g = grid_describe(type, elm_size, nd, dims, layout);
-  cudaError_t e = cudaMalloc(&g->alloc, g->alloc_bytes);
-  std::lock_guard<std::recursive_mutex> lk(rt().mu);
-  if (e == cudaErrorMemoryAllocation && g_work) {
-    cudaGetLastError();
-    work_release();
-    e = cudaMalloc(&g->alloc, g->alloc_bytes);
-  }
+  cudaError_t e = device_malloc(&g->alloc, g->alloc_bytes);
   if (e != cudaSuccess) {
     delete g;
     cudaGetLastError();
@@ -290,7 +319,10 @@ static psb_status grid_alloc(int type, int elm_size, int nd, const int *dims, in
     return cuda_status(e, "cudaMemset(grid)");
   }
   grid_attach(g);
-  g_grids++;
+  {
+    std::lock_guard<std::recursive_mutex> lk(g_work_mu);
+    g_grids++;
+  }
   *out = g;
   return PSB_OK;
 }
@@ -308,7 +340,7 @@ psb_status grid_alloc_pool(int type, const int *dims, cudaMemPool_t pool, cudaSt
   for (int i = 0; i < 3; i++)
     if (dims[i] <= 0) return set_status(PSB_ERR_INVALID);
   GridImpl *g = grid_describe(type, type_size(type), 3, dims, PSB_LAYOUT_PITCHED);
-  cudaError_t e = cudaMallocFromPoolAsync(&g->alloc, g->alloc_bytes, pool, s);
+  cudaError_t e = device_malloc_async(&g->alloc, g->alloc_bytes, pool, s);
   if (e == cudaSuccess) e = cudaMemsetAsync(g->alloc, 0, g->alloc_bytes, s);
   if (e != cudaSuccess) {
     if (g->alloc) cudaFreeAsync(g->alloc, s);
@@ -353,7 +385,7 @@ static void grid_free(GridImpl *g) {
   } else if (g->alloc) {
     cudaStreamSynchronize(rt().stream);
     PSB_FATAL(cudaFree(g->alloc));
-    std::lock_guard<std::recursive_mutex> lk(rt().mu);
+    std::lock_guard<std::recursive_mutex> lk(g_work_mu);
     if (--g_grids == 0) work_release();
   }
   g->magic = 0;

@@ -708,7 +708,7 @@ psb_status psb_server_create(size_t mem_budget_bytes, int max_slots, int mode, p
   if (e == cudaSuccess) e = cudaEventCreate(&S->ev0);
   if (e == cudaSuccess) e = cudaEventCreate(&S->ev1);
   if (e == cudaSuccess) e = cudaEventCreate(&S->ev_prev);
-  if (e == cudaSuccess) e = cudaMalloc(&S->d_norm, sizeof(double) * 2 * kNormBlocks);
+  if (e == cudaSuccess) e = device_malloc(&S->d_norm, sizeof(double) * 2 * kNormBlocks);
   if (e != cudaSuccess) {
     psb_status st = cuda_status(e, "psb_server_create");
     if (S->pool) cudaMemPoolDestroy(S->pool);

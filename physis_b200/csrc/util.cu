@@ -108,7 +108,7 @@ psb_status pitched_transfer(GridImpl *g, void *host, bool h2d, cudaStream_t s) {
   const GridView v = g->view();
   void *stage = nullptr;
   cudaMemPool_t pool = staging_pool();
-  if (pool && cudaMallocFromPoolAsync(&stage, bytes, pool, s) == cudaSuccess) {
+  if (pool && device_malloc_async(&stage, bytes, pool, s) == cudaSuccess) {
     const int64_t rows = (int64_t)v.n[1] * v.n[2];
     const int blocks = (int)std::max<int64_t>(1, std::min<int64_t>((rows + 7) / 8,
                                                                     (int64_t)rt().sm_count * 16));
@@ -201,7 +201,7 @@ psb_status user_transfer(GridImpl *g, void *host, bool h2d, cudaStream_t s) {
   cudaMemPool_t pool = staging_pool();
   if (!pool) return set_status(PSB_ERR_NOMEM);
   void *stage = nullptr;
-  PSB_TRY(cudaMallocFromPoolAsync(&stage, data_off + data, pool, s));
+  PSB_TRY(device_malloc_async(&stage, data_off + data, pool, s));
   unsigned char *base = (unsigned char *)stage;
   PSB_TRY(cudaMemcpyAsync(base, comps.data(), table, cudaMemcpyHostToDevice, s));
   if (h2d) PSB_TRY(cudaMemcpyAsync(base + data_off, host, data, cudaMemcpyHostToDevice, s));
@@ -226,7 +226,7 @@ psb_status pitched_stage_out(GridImpl *g, void **stage, cudaStream_t s) {
   *stage = nullptr;
   cudaMemPool_t pool = staging_pool();
   if (!pool) return set_status(PSB_ERR_NOMEM);
-  PSB_TRY(cudaMallocFromPoolAsync(stage, bytes, pool, s));
+  PSB_TRY(device_malloc_async(stage, bytes, pool, s));
   const int64_t rows = (int64_t)v.n[1] * v.n[2];
   const int blocks = (int)std::max<int64_t>(1, std::min<int64_t>((rows + 7) / 8,
                                                                   (int64_t)rt().sm_count * 16));

@@ -22,6 +22,7 @@ STUB = r"""
 namespace psb {
 psb_status set_status(psb_status s) { return s; }
 psb_status cuda_status(cudaError_t, const char *) { return PSB_ERR_CUDA; }
+cudaError_t device_malloc(void **p, size_t n) { *p = malloc(n); return cudaSuccess; }
 }  // namespace psb
 
 namespace psb {
