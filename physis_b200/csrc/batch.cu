@@ -912,15 +912,16 @@ static MemberTune member_tune(const BatchMemberHost &h) {
 // Sweeps per pass of a Himeno member whose bucket has no tune entry: two
 // when it is at least 120 points inside on every axis and the 64-wide tiles
 // of the two-sweep pass leave at most 15% of their columns outside its x
-// extent. Measured in the persistent batch on B200 (GLUPS, one sweep -> two):
-// cubes of 128 and 256 gain 11% and 5%; cubes of 32, 48, 64 and 96 lose
-// 39%, 12%, 10% and 18% (small members get short z chunks, so each pass
-// re-reads a larger share of halo planes; 96 wastes 27% of its tile columns).
-// With 16-byte pressure loads (HimenoRows) one sweep gained more: cubes of 112
-// to 160 now run 1 to 27% faster with it, 192 to 384 within 12% either way,
-// and a batch with one member on the two-sweep list beside others on the
-// one-sweep list took 4.24 ms against 3.18; the shipped table therefore keeps
-// one sweep up to buckets of 256.
+// extent. Persistent batch, ms per 20 steps, one sweep / two: cubes of 256
+// 2.92 / 2.29, 240 2.58 / 1.95, 224 1.99 / 1.72, 192 1.35 / 1.14, 176 1.20 /
+// 0.97, 128 0.54 / 0.50; cubes of 160 and 144, which waste 18 and 26% of the
+// columns, 0.81 / 1.08 and 0.78 / 0.85; (70, 70, 140) 0.24 / 0.30. Several
+// members on the two-sweep list gain more (eight cubes of 128 2.99 / 2.43).
+// One beside small members on the other lists gains from 240 on (3.12 / 2.79
+// at 256), loses 2 to 13% between 176 and 224 and 27% at 128: the two lists'
+// blocks share the SMs badly. The shipped table keeps one sweep in every bucket
+// of at most 128 in some extent; the bucket of 129 to 256 has no entry, because
+// both answers occur in it.
 static int default_sweeps(const BatchMemberHost &h) {
   const int *n = h.grids[0]->pub.dim;
   const int ix = n[0] - 2, iy = n[1] - 2, iz = n[2] - 2;
