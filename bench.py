@@ -477,7 +477,7 @@ def run_ours(args):
         tune = ps.autotune(kernel, ptype, dims) if args.tune else ps.tune_get(kernel, ptype, dims)
         if args.t_depth and kname == "diffusion7" and dt == np.float32:
             # pin the temporal depth of this shape (profiling)
-            tune = dict(tune, t_depth=args.t_depth)
+            tune = dict(tune, t_depth=0 if args.t_depth == 1 else 2)
             if args.t_depth == 2:
                 tune.update(impl=ps.IMPL_TMA, tile_x=128, tile_y=16)
             if args.z_chunk:

@@ -675,8 +675,12 @@ typedef struct {
   int tile_y;       /* points per CTA in y */
   int z_chunk;      /* planes per CTA work item */
   int stages;       /* pipelined planes in flight */
-  int t_depth;      /* steps per pass (1: single steps; 2: passes of two, for
-                     * a 7-point entry on tile_y 16 of up to four) */
+  int t_depth;      /* steps per pass in a run of two maps that swap two grids.
+                     * 7-point: 1 whatever the library estimates fastest (as
+                     * without an entry), 2 passes of two steps, 0 single
+                     * steps only. Himeno: 1 single sweeps, 2 two per pass
+                     * (without an entry: two). Maps run alone take single
+                     * steps of the other fields' shape. */
 } psb_tune_config;
 psb_status psb_autotune(int kernel_id, int type, const PSIndex *dims, int force,
                         psb_tune_config *cfg);

@@ -348,11 +348,9 @@ struct PipePlan {
   int passes() const { return count[2] + count[3] + count[4]; }
 };
 
-// False: the run keeps single steps. A tune entry of a clamped float shape
-// decides: t_depth 1 keeps single steps, t_depth 2 two-step passes only, and
-// t_depth 2 on tile_y 16 whatever passes are estimated fastest, which is also
-// the rule without an entry and for the other kinds (the tuner records only
-// single-step shapes for them).
+// False: the run keeps single steps. A tune entry of the shape pins them with
+// t_depth 0 or the plain kernel, and passes of two steps with t_depth 2;
+// otherwise, as without an entry, whatever is estimated fastest.
 static bool pipe_plan(MapImpl **ms, int iter, PipePlan *plan) {
   const Runtime &r = rt();
   const GridImpl *A = ms[0]->grids[0];
@@ -361,9 +359,9 @@ static bool pipe_plan(MapImpl **ms, int iter, PipePlan *plan) {
   const bool per = ms[0]->kernel_id == PSB_KERNEL_DIFFUSION7_PERIODIC;
   bool free_choice = true;
   psb_tune_config cfg;
-  if (tune_find(ms[0]->kernel_id, dbl ? PS_DOUBLE : PS_FLOAT, n, &cfg) && !per && !dbl) {
-    if (cfg.t_depth != 2) return false;
-    free_choice = cfg.tile_y == 16;
+  if (tune_find(ms[0]->kernel_id, dbl ? PS_DOUBLE : PS_FLOAT, n, &cfg)) {
+    if (cfg.t_depth == 0 || (cfg.impl == PSB_IMPL_PLAIN && r.impl != PSB_IMPL_TMA)) return false;
+    free_choice = cfg.t_depth != 2;
   }
   const int steps = 2 * iter - 1;  // before the last one
   double t4 = -1, t3 = -1, t2 = -1;

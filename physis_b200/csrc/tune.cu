@@ -214,29 +214,17 @@ static double time_config(MapImpl &m, const psb_tune_config &cfg, int reps) {
   cudaEventCreate(&b);
   double best = -1;
   int64_t launches = 0;
-  // A 7-point entry with t_depth 2 runs passes of two steps, or on tile_y 16
-  // passes of four where the rule has a shape for them.
-  PipeConfig pass{};
-  if (m.kernel_id != PSB_KERNEL_HIMENO19 && cfg.t_depth == 2) {
-    double cost = -1;
-    const int *n = m.grids[0]->pub.dim;
-    if (cfg.tile_y == 16) pass = diff7_pipe_choose(4, false, false, r.fp_mode == PSB_FP_FMA, n, &cost);
-    if (cost < 0) pass = diff7_pipe_choose(2, false, false, r.fp_mode == PSB_FP_FMA, n, &cost);
-    if (cost < 0) return -1;
-  }
   for (int round = 0; round < 4; round++) {
     cudaEventRecord(a, r.stream);
     for (int i = 0; i < reps; i++) {
-      // Two-step (temporally blocked) candidates advance two steps per launch.
+      // A two-sweep Himeno candidate advances two sweeps per launch.
       psb_status st;
       if (m.kernel_id == PSB_KERNEL_HIMENO19)
         st = cfg.t_depth == 2 ? himeno_tb2_launch(m, m, m.grids[0], m.grids[1], cfg.z_chunk,
                                                   false, false, r.stream, &launches)
                               : himeno_launch(m, cfg, r.stream, &launches);
       else
-        st = cfg.t_depth == 2
-                 ? diff7_pipe_launch(m, m.grids[0], m.grids[1], pass, r.stream, &launches)
-                 : diffusion7_launch(m, cfg, r.stream, &launches);
+        st = diffusion7_launch(m, cfg, r.stream, &launches);
       if (st != PSB_OK) {
         cudaEventDestroy(a);
         cudaEventDestroy(b);
@@ -251,7 +239,7 @@ static double time_config(MapImpl &m, const psb_tune_config &cfg, int reps) {
     }
     float ms = 0;
     cudaEventElapsedTime(&ms, a, b);
-    ms /= pass.ns ? pass.ns : cfg.t_depth == 2 ? 2 : 1;  // per step
+    ms /= cfg.t_depth == 2 ? 2 : 1;  // per step
     if (round > 0 && (best < 0 || ms / reps < best)) best = ms / reps;  // round 0 warms up
   }
   cudaEventDestroy(a);
@@ -335,6 +323,8 @@ psb_status psb_autotune(int kernel_id, int type, const PSIndex *dims, int force,
   cudaStreamSynchronize(r.stream);
   int64_t pts = (int64_t)dims[0] * dims[1] * dims[2];
   int reps = (int)std::max<int64_t>(3, std::min<int64_t>(50, 400000000LL / std::max<int64_t>(pts, 1)));
+  // 7-point kernels: the shapes of single steps (t_depth 1 leaves passes of
+  // several steps to the estimate of a run).
   std::vector<psb_tune_config> cands;
   psb_tune_config plain = default_config(kernel_id, type, (const int *)dims);
   plain.impl = PSB_IMPL_PLAIN;
@@ -359,21 +349,6 @@ psb_status psb_autotune(int kernel_id, int type, const PSIndex *dims, int force,
           c.t_depth = 1;
           cands.push_back(c);
         }
-  // Passes of several steps (clamped float 7-point): the rule's (tile_y 16)
-  // and two-step passes only (tile_y 8). The fields are a valid single-step
-  // configuration too, for maps run alone.
-  if (kernel_id == PSB_KERNEL_DIFFUSION7 && type == PS_FLOAT && dims[0] >= 4 && dims[1] >= 4 &&
-      dims[2] >= 4)
-    for (int ty : {16, 8}) {
-      psb_tune_config c;
-      c.impl = PSB_IMPL_TMA;
-      c.tile_x = 128;
-      c.tile_y = ty;
-      c.z_chunk = 32;
-      c.stages = 6;
-      c.t_depth = 2;
-      cands.push_back(c);
-    }
   // Himeno, two sweeps per pass (64 x 12 tiles; the single-sweep fields of
   // the entry are the default shape, used for maps run alone).
   if (kernel_id == PSB_KERNEL_HIMENO19)
