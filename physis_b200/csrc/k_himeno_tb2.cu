@@ -197,7 +197,8 @@ bool himeno_tb2_pair(MapImpl **ms, int n) {
   if (n != 2) return false;
   const MapImpl &a = *ms[0], &b = *ms[1];
   if (a.kernel_id != PSB_KERNEL_HIMENO19 || b.kernel_id != PSB_KERNEL_HIMENO19) return false;
-  if (a.color != -1 || b.color != -1 || a.params[0] != b.params[0]) return false;
+  if (a.color != -1 || b.color != -1) return false;
+  if (memcmp(a.params, b.params, sizeof(double)) != 0) return false;  // (0 is not -0)
   if (b.grids[0] != a.grids[1] || b.grids[1] != a.grids[0] || a.grids[0] == a.grids[1])
     return false;
   if (memcmp(&a.dom, &b.dom, sizeof(a.dom)) != 0) return false;

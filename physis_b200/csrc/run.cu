@@ -320,8 +320,7 @@ static bool pipe_pair(MapImpl **ms, int n) {
   if (a.kernel_id != PSB_KERNEL_DIFFUSION7 && a.kernel_id != PSB_KERNEL_DIFFUSION7_PERIODIC)
     return false;
   if (b.kernel_id != a.kernel_id || a.color != -1 || b.color != -1) return false;
-  for (int i = 0; i < 7; i++)
-    if (a.params[i] != b.params[i]) return false;
+  if (memcmp(a.params, b.params, 7 * sizeof(double)) != 0) return false;  // (0 is not -0)
   GridImpl *A = a.grids[0], *B = a.grids[1];
   if (b.grids[0] != B || b.grids[1] != A || A == B) return false;
   for (GridImpl *g : {A, B}) {
