@@ -310,30 +310,34 @@ void maps_forget_grid(const GridImpl *g) {
   }
 }
 
-// The pattern that passes of several steps apply to: PSStencilRun(m1, m2,
-// iter) with m1: A -> B and m2: B -> A the same 7-point map (clamped or
-// periodic) over the whole of two pitched grids of at least four points a
-// side (a periodic pass wraps up to two).
-static bool pipe_pair(MapImpl **ms, int n) {
-  if (n != 2) return false;
-  const MapImpl &a = *ms[0], &b = *ms[1];
-  if (a.kernel_id != PSB_KERNEL_DIFFUSION7 && a.kernel_id != PSB_KERNEL_DIFFUSION7_PERIODIC)
+// A 7-point map (clamped or periodic) that passes of several steps apply to:
+// over the whole of two pitched grids of at least four points a side (a periodic
+// pass wraps up to two).
+static bool pipe_map(const MapImpl &m) {
+  if (m.kernel_id != PSB_KERNEL_DIFFUSION7 && m.kernel_id != PSB_KERNEL_DIFFUSION7_PERIODIC)
     return false;
-  if (b.kernel_id != a.kernel_id || a.color != -1 || b.color != -1) return false;
-  if (memcmp(a.params, b.params, 7 * sizeof(double)) != 0) return false;  // (0 is not -0)
-  GridImpl *A = a.grids[0], *B = a.grids[1];
-  if (b.grids[0] != B || b.grids[1] != A || A == B) return false;
-  for (GridImpl *g : {A, B}) {
+  const GridImpl *A = m.grids[0];
+  if (m.color != -1 || A == m.grids[1]) return false;
+  for (const GridImpl *g : {A, (const GridImpl *)m.grids[1]}) {
     if (g->layout != PSB_LAYOUT_PITCHED || g->type != A->type || !tma_eligible(g) ||
         (g->type != PS_FLOAT && g->type != PS_DOUBLE))
       return false;
     for (int i = 0; i < 3; i++)
       if (g->pub.dim[i] != A->pub.dim[i] || g->pub.dim[i] < 4) return false;
   }
-  for (const MapImpl *m : {&a, &b})
-    for (int i = 0; i < 3; i++)
-      if (m->dom.local_min[i] != 0 || m->dom.local_max[i] != A->pub.dim[i]) return false;
+  for (int i = 0; i < 3; i++)
+    if (m.dom.local_min[i] != 0 || m.dom.local_max[i] != A->pub.dim[i]) return false;
   return true;
+}
+
+// The runs that advance several steps per pass: PSStencilRun(m1, m2, iter) with
+// m1: A -> B and m2: B -> A the same such map.
+static bool pipe_pair(MapImpl **ms, int n) {
+  if (n != 2) return false;
+  const MapImpl &a = *ms[0], &b = *ms[1];
+  if (!pipe_map(a) || !pipe_map(b) || b.kernel_id != a.kernel_id) return false;
+  if (memcmp(a.params, b.params, 7 * sizeof(double)) != 0) return false;  // (0 is not -0)
+  return b.grids[0] == a.grids[1] && b.grids[1] == a.grids[0];
 }
 
 // How a run of `iter` pairs is cut: passes of four, three and two steps and
@@ -405,18 +409,24 @@ static bool pipe_plan(MapImpl **ms, int iter, PipePlan *plan) {
   return plan->passes() > 0;
 }
 
+// One pass of map m from grid in to grid out, with the halo it reads and the
+// state of the one it leaves.
+static psb_status pipe_pass(MapImpl &m, GridImpl *in, GridImpl *out, const PipeConfig &cfg,
+                            int64_t *launches) {
+  const bool per = m.kernel_id == PSB_KERNEL_DIFFUSION7_PERIODIC;
+  if (per && in->ghost_valid != PSB_BOUNDARY_PERIODIC && in->ghost_valid != kGhostXY)
+    PSB_CHECK(launch_halo_fill(in, PSB_BOUNDARY_PERIODIC, rt().stream));
+  PSB_CHECK(diff7_pipe_launch(m, in, out, cfg, rt().stream, launches));
+  out->ghost_valid = per ? kGhostXY : PSB_BOUNDARY_NONE;
+  return PSB_OK;
+}
+
 static psb_status run_pipe(MapImpl **ms, const PipePlan &plan, int64_t *launches) {
-  Runtime &r = rt();
-  const bool per = ms[0]->kernel_id == PSB_KERNEL_DIFFUSION7_PERIODIC;
   GridImpl *g[2] = {ms[0]->grids[0], ms[0]->grids[1]};
   int at = 0;  // the grid that holds the state
   for (int i = 0; i < plan.passes(); i++) {
     const int ns = i < plan.count[4] ? 4 : i < plan.count[4] + plan.count[3] ? 3 : 2;
-    GridImpl *in = g[at], *out = g[at ^ 1];
-    if (per && in->ghost_valid != PSB_BOUNDARY_PERIODIC && in->ghost_valid != kGhostXY)
-      PSB_CHECK(launch_halo_fill(in, PSB_BOUNDARY_PERIODIC, r.stream));
-    PSB_CHECK(diff7_pipe_launch(*ms[0], in, out, plan.pass[ns], r.stream, launches));
-    out->ghost_valid = per ? kGhostXY : PSB_BOUNDARY_NONE;
+    PSB_CHECK(pipe_pass(*ms[0], g[at], g[at ^ 1], plan.pass[ns], launches));
     at ^= 1;
   }
   for (int i = 0; i <= plan.count[1]; i++) {
@@ -849,6 +859,34 @@ psb_status psb_stencil_run(const PSStencil *maps, int nmaps, int iter) {
     if (!ms[i]) return set_status(PSB_ERR_INVALID);
   }
   return run_maps(ms, nmaps, iter);
+}
+
+// One pass of `steps` steps of a 7-point map from its input to its output grid, in
+// the shape that runs would take, or with the given threads a block, lanes a row
+// (2^lanes_shift) and z chunk (threads > 0). Runs choose depth and shape by
+// estimated time, which leaves most combinations to large grids; the tests call
+// this to reach every one of them (not part of the public interface).
+psb_status psb_diff7_pass(PSStencil h, int steps, int threads, int lanes_shift, int z_chunk) {
+  std::lock_guard<std::recursive_mutex> lk(rt().mu);
+  MapImpl *m = map_of(h);
+  if (!m || steps < 2 || steps > 4) return set_status(PSB_ERR_INVALID);
+  PSB_CHECK(check_map(*m));
+  const bool per = m->kernel_id == PSB_KERNEL_DIFFUSION7_PERIODIC;
+  if (!pipe_map(*m) || (per && steps > 2)) return set_status(PSB_ERR_UNSUPPORTED);
+  PipeConfig cfg{steps, steps > 2 ? 2 : 4, threads, lanes_shift, z_chunk, 4};
+  if (threads > 0) {
+    if (lanes_shift < 3 || lanes_shift > 5 || z_chunk < 1) return set_status(PSB_ERR_INVALID);
+  } else {
+    double cost = -1;
+    cfg = diff7_pipe_choose(steps, m->grids[0]->type == PS_DOUBLE, per,
+                            rt().fp_mode == PSB_FP_FMA, m->grids[0]->pub.dim, &cost);
+    if (cost < 0) return set_status(PSB_ERR_UNSUPPORTED);
+  }
+  int64_t launches = 0;
+  legacy_join_in();
+  PSB_TRY(cudaEventRecord(rt().ev_start, rt().stream));
+  PSB_CHECK(pipe_pass(*m, m->grids[0], m->grids[1], cfg, &launches));
+  return finish_run(launches);
 }
 
 psb_status psb_stencil_free(PSStencil s) {
