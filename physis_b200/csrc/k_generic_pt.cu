@@ -28,24 +28,10 @@
 #include <string>
 
 #include "internal.h"
+#include "k_generic_pt.cuh"
 
 namespace psb {
 namespace {
-
-// The host's copy of GpArgs (k_generic_pt.cuh), which only the run-time
-// compiled kernel includes.
-struct GpArgs {
-  GridView g[PSB_MAX_GRIDS];
-  double a[PSB_MAX_TERMS], b[PSB_MAX_TERMS], post;
-  float a32[PSB_MAX_TERMS], b32[PSB_MAX_TERMS], post32;
-  Dom3 d;
-  int color;
-  int tx_shift;
-  int tiles_x, tiles_y;
-  unsigned mul_x, mul_y;
-  int shift_x, shift_y;
-};
-constexpr int kGpThreads = 256;
 
 // b / d as (b * mul) >> shift, exact for 0 <= b < 2^31: with 2^(l-1) < d <= 2^l
 // and mul = floor(2^(31+l) / d) + 1, b * mul / 2^(31+l) exceeds b / d by less
@@ -152,6 +138,8 @@ std::string source_of(const psb_generic_stencil &d, const GpShape &sh) {
   bool slim = d.nterms <= 8 && d.accum_type == PS_FLOAT;
   for (int i = 0; i < d.ngrids; i++) slim = slim && d.grid_type[i] == PS_FLOAT;
   std::string s = std::string("#include \"k_generic_pt.cuh\"\n"
+                              "static_assert(sizeof(psb::GpArgs) == " +
+                              std::to_string(sizeof(GpArgs)) + ", \"as the host fills it\");\n"
                               "extern \"C\" __global__ void __launch_bounds__(256") +
                   (slim ? ", 8" : "") + ") "
                   "psb_generic_points(const __grid_constant__ psb::GpArgs q) {\n"

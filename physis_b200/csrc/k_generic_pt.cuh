@@ -1,6 +1,7 @@
 // Device side of the compiled point kernel of a generic stencil
-// (k_generic_pt.cu writes the kernel's source for one table). Included only
-// by that source, so it compiles under the run-time compiler.
+// (k_generic_pt.cu writes the kernel's source for one table). Included by
+// that source, so it compiles under the run-time compiler, and by its writer,
+// which fills GpArgs.
 #pragma once
 
 #include "device.cuh"
