@@ -466,9 +466,13 @@ psb_status psb_generic_last_impl(int *impl);
  * the map first runs --
  * the reference's translator likewise emits one kernel per stencil
  * (translator/cuda_translator.cc:615-869) -- and cached per process for
- * every table of the same shape (coefficients are launch arguments). Same
- * arithmetic, same results; without NVRTC or the library's device headers
- * (csrc/ beside lib/, or $PHYSIS_B200_CSRC) the interpreting kernel runs. */
+ * every table of the same shape (coefficients are launch arguments); so are
+ * tables off the TMA path, for the thread-per-point kernel. Compiling takes
+ * 0.04 s (a few terms on a small grid) to 0.5 s (32 terms on a large one) at
+ * the first application; a program that applies a table only a few times may
+ * want psb_set_generic_compile(0). Same arithmetic, same results; without
+ * NVRTC or the library's device headers (csrc/ beside lib/, or
+ * $PHYSIS_B200_CSRC) the interpreting kernel runs. */
 psb_status psb_generic_last_compiled(int *compiled);
 /* Run-time compilation of generic tables on (1, the default unless
  * $PHYSIS_B200_GENERIC_COMPILE=0) or off (0). */

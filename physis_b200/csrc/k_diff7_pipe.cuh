@@ -13,7 +13,7 @@
 // barrier per turn. Input planes stream through a ring of TMA boxes issued
 // S - 2 turns ahead.
 //
-// What bounds it: instruction issue (59-60% of the slots at 512^3; the input
+// What bounds it: instruction issue (66% of the slots at 512^3; the input
 // is read and the output written once for NS steps, so DRAM is not the
 // limit). Hence the shape: R rows a thread, because the exchange (two loads,
 // two stores, two shuffles a row) is paid per thread and row group, not per

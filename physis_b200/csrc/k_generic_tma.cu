@@ -374,7 +374,8 @@ static psb_status gt_launch(MapImpl &m, const psb_generic_stencil &desc, const G
   GtGeom geo;
   GtMaps maps;
   int64_t nblocks = 0;
-  // Blocks an SM holds: the kernels' launch bounds.
+  // The residency that gt_zchunk's constants were fitted with: the launch bounds of
+  // the window forms (the plane form's promise three blocks an SM for float too).
   if (gt_geometry<T>(m, p, og, d, sizeof(T) == 4 ? 4 : 3, false, geo, maps, &nblocks) != PSB_OK)
     return PSB_ERR_UNSUPPORTED;
   GtTable tab;
@@ -479,6 +480,8 @@ static psb_status staged_run(MapImpl &m, psb_compiled_staged fn, const GtPlan &p
   GtGeom geo;
   GtMaps maps;
   int64_t nblocks = 0;
+  // Three blocks an SM, as fitted: the launch bounds of functions of up to fourteen
+  // reads (longer ones promise two).
   if (gt_geometry<T>(m, p, og, d, 3, true, geo, maps, &nblocks) != PSB_OK)
     return PSB_ERR_UNSUPPORTED;
   const size_t smem = 128 + 512 + (size_t)geo.stages * geo.stage_bytes;

@@ -140,7 +140,7 @@ __global__ void __launch_bounds__(kHtThreads, 1)
   // CTA adds all partials in index order into the sweep's map history. All
   // consumer warps arrive here, a timed-out one too.
   constexpr int nct = 32 * (kHtW1 + kHtW2);
-  const int cw = warp - 1;  // consumer warp 0..8
+  const int cw = warp - 1;  // stage-1 warps 0..6, stage-2 warps 7..12
   if (bad && lane == 0) {
     atomicExch(&flags[1], 1);
     atomicExch(err, 1);
@@ -166,7 +166,7 @@ __global__ void __launch_bounds__(kHtThreads, 1)
   consumer_bar(nct);
   if (!flags[0]) return;
   __threadfence();
-  // Consumer warps 0..4 sum sweep 1, warps 5..8 sweep 2.
+  // The stage-1 warps sum sweep 1, the stage-2 warps sweep 2.
   const bool first = cw < kHtW1;
   const Residual &RS = first ? res1 : res2;
   const int tg = first ? tid - 32 : tid - 32 - 32 * kHtW1;

@@ -33,9 +33,10 @@
 // 257 x 257 x 513, us per sweep: 272 with eight rows and planes read from the
 // rings; 253 with the edge warp; 232 with the planes in registers; 208 released
 // early, 202 with five coefficient stages; 184 with twelve rows (0.78 of the
-// measured peak for the pass's 28 B per update). Fourteen rows need 17 warps,
-// which leaves 96 registers and spills (458); two points a thread instead of
-// four changes nothing; x neighbours by shuffle cost 8% (a longer chain).
+// measured peak for the pass's 28 B per update). It spills 68 bytes a thread, at
+// 128 registers. Fourteen rows need 17 warps, which leave 96 registers, and spill
+// far more (458); two points a thread instead of four changes nothing; x
+// neighbours by shuffle cost 8% (a longer chain).
 #pragma once
 
 #include "k_himeno.cuh"
