@@ -35,7 +35,7 @@ __global__ void __launch_bounds__(256) k_generic(const GenTable *__restrict__ ta
     for (int i = tid; i < words; i += nt) dst[i] = src[i];
   }
   __syncthreads();
-  const int p[3] = {d.lo[0] + (int)(blockIdx.x * blockDim.x + threadIdx.x),
+  const int p[3] = {gen_point(d.lo[0], d.hi[0], blockIdx.x * blockDim.x + threadIdx.x),
                     d.lo[1] + (int)(blockIdx.y * blockDim.y + threadIdx.y),
                     d.lo[2] + (int)(blockIdx.z * blockDim.z + threadIdx.z)};
   if (p[0] >= d.hi[0] || p[1] >= d.hi[1] || p[2] >= d.hi[2]) return;
@@ -174,8 +174,8 @@ __global__ void __launch_bounds__(256) k_generic_reduce(const GenTable *__restri
     int p[3];
     p[1] = d.lo[1] + (int)(r % ry);
     p[2] = d.lo[2] + (int)(r / ry);
-    for (int x = lane; x < rx; x += 32) {
-      p[0] = d.lo[0] + x;
+    for (int64_t x = lane; x < rx; x += 32) {  // (x + 32 may exceed the largest int)
+      p[0] = d.lo[0] + (int)x;
       A acc = 0;
       for (int i = 0; i < t.nterms; i++) {
         A v = xmul(gen_factor<A>(G, t.a[i], p), gen_factor<A>(G, t.b[i], p));

@@ -46,6 +46,12 @@ __device__ __forceinline__ int64_t gen_offset(const GridView &g, const int *axes
   return off;
 }
 
+// The point `i` from lo in [lo, hi), or hi where there is none: i covers the rest
+// of the last block too, so lo + i may lie beyond the largest int.
+__host__ __device__ __forceinline__ int gen_point(int lo, int hi, unsigned i) {
+  return i < (unsigned)hi - (unsigned)lo ? (int)((unsigned)lo + i) : hi;
+}
+
 template <typename A>
 __device__ __forceinline__ A gen_factor(const GenGrids &G, const GenFactor &f, const int *p) {
   if (f.grid < 0) return (A)f.c;

@@ -24,6 +24,7 @@
 // Arithmetic and order are those of k_generic, so results are bit-identical
 // (a factor that is the constant 1 is not multiplied: x * 1 == x).
 #include <algorithm>
+#include <climits>
 #include <cstring>
 #include <string>
 
@@ -201,12 +202,16 @@ std::string key_of(const psb_generic_stencil &d, const GpShape &sh) {
 }  // namespace
 
 // PSB_ERR_UNSUPPORTED when the map keeps k_generic: a written grid that does
-// not follow the domain's axes one to one, no run-time compiler, or a kernel
-// that is not compiled yet while the stream is being captured.
+// not follow the domain's axes one to one, columns near the largest int, no
+// run-time compiler, or a kernel that is not compiled yet while the stream is
+// being captured.
 psb_status generic_points_launch(MapImpl &m, const GenericDesc &gd, int color, cudaStream_t s,
                                  int64_t *launches) {
   const psb_generic_stencil &d = gd.host;
   if (!generic_compile_on()) return PSB_ERR_UNSUPPORTED;
+  // The last block's columns past the domain must be ints too (a check in the
+  // kernel costs every point of a short table).
+  if (m.dom.local_max[0] > INT_MAX - 2 * kGpThreads) return PSB_ERR_UNSUPPORTED;
   for (int k = 0; k < 3; k++)
     if (d.grid_axes[d.out_grid][k] != (k < d.ndims ? k : -1)) return PSB_ERR_UNSUPPORTED;
   for (int i = 0; i < d.ngrids; i++)  // axes listed from the first, without gaps
