@@ -932,9 +932,13 @@ static int default_sweeps(const BatchMemberHost &h) {
 
 // Work list of a member: 0 diffusion, 1 Himeno one sweep per item, 2 Himeno
 // up to two sweeps per item (when its tune entry or trial says so, or, with
-// neither, default_sweeps; and it runs at least two steps).
+// neither, default_sweeps; and it runs at least two steps, with no coefficient
+// that is one of its pressure grids: a pass reads coefficients once for both
+// sweeps).
 static int member_group(const BatchMemberHost &h, const MemberTune &mt, int steps) {
   if (h.kind != BK_HIMENO) return 0;
+  for (int i = 2; i < 14; i++)
+    if (h.grids[i] == h.grids[0] || h.grids[i] == h.grids[1]) return 1;
   const int td = mt.tuned || mt.forced ? mt.td : default_sweeps(h);
   return td == 2 && steps >= 2 ? 2 : 1;
 }
