@@ -798,6 +798,8 @@ struct psb_batch {
   std::vector<std::vector<int>> passes;  // group-2 members: local step of each pass
   int *d_pass = nullptr;
   size_t cap_pass = 0;
+  int *d_rims = nullptr;  // batch_check_rims: one word per member that it looks at
+  size_t cap_rims = 0;
   bool built = false;
   cudaGraphExec_t graph = nullptr;
   cudaStream_t side = nullptr, side2 = nullptr;  // streams of the second and third work lists
@@ -830,6 +832,9 @@ static void batch_release_device(psb_batch *b) {
   cudaFree(b->d_pass);
   b->d_pass = nullptr;
   b->cap_pass = 0;
+  cudaFree(b->d_rims);
+  b->d_rims = nullptr;
+  b->cap_rims = 0;
   b->d_members = nullptr;
   b->d_tmaps = nullptr;
   b->d_partials = nullptr;
@@ -934,13 +939,18 @@ static int default_sweeps(const BatchMemberHost &h) {
 // up to two sweeps per item (when its tune entry or trial says so, or, with
 // neither, default_sweeps; and it runs at least two steps, with no coefficient
 // that is one of its pressure grids: a pass reads coefficients once for both
-// sweeps).
+// sweeps. Nor where those two hold different values around the domain: a pass
+// takes its input's for both sweeps and leaves out every other grid).
+static bool two_sweep_member(const BatchMemberHost &h, const MemberTune &mt, int steps) {
+  if (h.kind != BK_HIMENO || steps < 2) return false;
+  for (int i = 2; i < 14; i++)
+    if (h.grids[i] == h.grids[0] || h.grids[i] == h.grids[1]) return false;
+  return (mt.tuned || mt.forced ? mt.td : default_sweeps(h)) == 2;
+}
+
 static int member_group(const BatchMemberHost &h, const MemberTune &mt, int steps) {
   if (h.kind != BK_HIMENO) return 0;
-  for (int i = 2; i < 14; i++)
-    if (h.grids[i] == h.grids[0] || h.grids[i] == h.grids[1]) return 1;
-  const int td = mt.tuned || mt.forced ? mt.td : default_sweeps(h);
-  return td == 2 && steps >= 2 ? 2 : 1;
+  return two_sweep_member(h, mt, steps) && !h.rims_differ ? 2 : 1;
 }
 
 // Passes of a group-2 member: from each local step s (global step0 + s) two
@@ -1542,6 +1552,39 @@ static psb_status batch_run_loop(psb_batch *b, int impl, int64_t *launches) {
   return st;
 }
 
+// Which members that would run two sweeps per item have different values around
+// the domains of their two pressure grids now; a change ends the work lists built
+// before. (The server's requests get the same values in both.)
+static psb_status batch_check_rims(psb_batch *b) {
+  std::vector<int> who, differ;
+  for (int i = 0; i < (int)b->hm.size(); i++)
+    if (two_sweep_member(b->hm[i], member_tune(b->hm[i]), b->hm[i].steps)) who.push_back(i);
+  if (who.empty()) return PSB_OK;
+  cudaStream_t s = rt().stream;
+  differ.resize(who.size());
+  const size_t bytes = sizeof(int) * who.size();
+  PSB_CHECK(dev_reserve(&b->d_rims, &b->cap_rims, bytes));
+  PSB_TRY(cudaMemsetAsync(b->d_rims, 0, bytes, s));
+  for (size_t k = 0; k < who.size(); k++) {
+    const BatchMemberHost &h = b->hm[who[k]];
+    Dom3 d;
+    for (int i = 0; i < 3; i++) {
+      d.lo[i] = 1;
+      d.hi[i] = h.grids[0]->pub.dim[i] - 1;
+    }
+    PSB_CHECK(himeno_rim_compare(h.grids[0], h.grids[1], d, b->d_rims + k, s));
+  }
+  PSB_TRY(cudaMemcpyAsync(differ.data(), b->d_rims, bytes, cudaMemcpyDeviceToHost, s));
+  PSB_TRY(cudaStreamSynchronize(s));
+  for (size_t k = 0; k < who.size(); k++) {
+    bool &was = b->hm[who[k]].rims_differ;
+    if (was == (differ[k] != 0)) continue;
+    was = differ[k] != 0;
+    batch_invalidate(b);
+  }
+  return PSB_OK;
+}
+
 }  // namespace psb
 
 extern "C" {
@@ -1605,6 +1648,7 @@ psb_status psb_batch_run(psb_batch *b, int mode) {
         h.grids[0]->ghost_valid != kGhostFaces)
       PSB_CHECK(launch_halo_fill(h.grids[0], PSB_BOUNDARY_PERIODIC, r.stream));
   if (mode == 0 || mode == 1) {
+    PSB_CHECK(batch_check_rims(b));
     if (!b->built) {
       std::vector<int> steps, step0;
       for (auto &h : b->hm) {

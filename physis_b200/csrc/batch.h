@@ -24,6 +24,7 @@ struct BatchMemberHost {
   int force_zc = 0;        // autotuner trials: planes per item (0: choose)
   int force_td = 0;        // autotuner trials: Himeno sweeps per pass, 1 or 2 (0: choose)
   int cur0 = 0;            // which of grids[0], grids[1] holds the state at the first step
+  bool rims_differ = false;  // Himeno: the two hold different values around the domain
 };
 
 }  // namespace psb

@@ -219,6 +219,10 @@ int himeno_tb2_chunk(const __PSDomain &dom);  // z chunk of the pass over a doma
 // The cells around map m's domain from its input grid to dst, compared with its
 // output grid's on the way (Runtime::rim_run).
 psb_status himeno_rim_copy(const MapImpl &m, GridImpl *dst, cudaStream_t s, int64_t *launches);
+// *differs = 1 (else left alone) where two pressure grids' cells around domain d
+// hold different values.
+psb_status himeno_rim_compare(const GridImpl *a, const GridImpl *b, const Dom3 &d, int *differs,
+                              cudaStream_t s);
 psb_status himeno_tb2_launch(MapImpl &m1, MapImpl &m2, GridImpl *in, GridImpl *out,
                              int zchunk, bool rims, bool last, cudaStream_t s, int64_t *launches);
 psb_status generic_tma_launch(MapImpl &m, const GenericDesc &gd, int color, cudaStream_t s,

@@ -259,8 +259,8 @@ static psb_status ht_residual(MapImpl &m, int nblocks, Residual *r) {
   return PSB_OK;
 }
 
-// The cells around the domain (one deep, with edges and corners), src -> dst;
-// *differs = run where other holds another value in one of them.
+// The cells around the domain (one deep, with edges and corners), src -> dst (or
+// compared only); *differs = run where other holds another value in one of them.
 __global__ void k_himeno_rim(const float *src, const float *other, float *dst, int64_t sy,
                              int64_t sz, Dom3 d, int *differs, int run) {
   const int ex = d.hi[0] - d.lo[0] + 2, ey = d.hi[1] - d.lo[1] + 2, ez = d.hi[2] - d.lo[2] + 2;
@@ -280,29 +280,38 @@ __global__ void k_himeno_rim(const float *src, const float *other, float *dst, i
     }
     const int64_t o = (x + d.lo[0] - 1) + (y + d.lo[1] - 1) * sy + (z + d.lo[2] - 1) * sz;
     const float v = src[o];
-    dst[o] = v;
+    if (dst) dst[o] = v;
     if (__float_as_int(v) != __float_as_int(other[o])) *differs = run;
   }
 }
 
+static psb_status rim_launch(const GridImpl *src, const GridImpl *other, GridImpl *dst,
+                             const Dom3 &d, int *differs, int run, cudaStream_t s) {
+  int64_t e[3];
+  for (int i = 0; i < 3; i++) e[i] = d.hi[i] - d.lo[i] + 2;
+  const int64_t n = 2 * (e[0] * e[1] + e[0] * e[2] + e[1] * e[2]);
+  k_himeno_rim<<<(unsigned)std::min<int64_t>((n + 255) / 256, 8 * rt().sm_count), 256, 0, s>>>(
+      (const float *)src->view().origin, (const float *)other->view().origin,
+      dst ? (float *)dst->view().origin : nullptr, src->sy, src->sz, d, differs, run);
+  PSB_TRY(cudaGetLastError());
+  return PSB_OK;
+}
+
 psb_status himeno_rim_copy(const MapImpl &m, GridImpl *dst, cudaStream_t s, int64_t *launches) {
   Runtime &r = rt();
-  const GridImpl *src = m.grids[0], *other = m.grids[1];
   r.rim_run = r.rim_run == INT_MAX ? 1 : r.rim_run + 1;
   Dom3 d;
-  int64_t e[3];
   for (int i = 0; i < 3; i++) {
     d.lo[i] = m.dom.local_min[i];
     d.hi[i] = m.dom.local_max[i];
-    e[i] = d.hi[i] - d.lo[i] + 2;
   }
-  const int64_t n = 2 * (e[0] * e[1] + e[0] * e[2] + e[1] * e[2]);
-  k_himeno_rim<<<(unsigned)std::min<int64_t>((n + 255) / 256, 8 * r.sm_count), 256, 0, s>>>(
-      (const float *)src->view().origin, (const float *)other->view().origin,
-      (float *)dst->view().origin, src->sy, src->sz, d, r.d_error + 2, r.rim_run);
   (*launches)++;
-  PSB_TRY(cudaGetLastError());
-  return PSB_OK;
+  return rim_launch(m.grids[0], m.grids[1], dst, d, r.d_error + 2, r.rim_run, s);
+}
+
+psb_status himeno_rim_compare(const GridImpl *a, const GridImpl *b, const Dom3 &d, int *differs,
+                              cudaStream_t s) {
+  return rim_launch(a, b, nullptr, d, differs, 1, s);
 }
 
 // Two sweeps, in -> out: the first is map m1's sweep, the second m2's (their
