@@ -467,15 +467,15 @@ psb_status psb_generic_last_impl(int *impl);
  * the reference's translator likewise emits one kernel per stencil
  * (translator/cuda_translator.cc:615-869) -- and cached per process for
  * every table of the same shape (coefficients are launch arguments); so are
- * tables off the TMA path, for the thread-per-point kernel. Compiling takes
- * 0.04 s (a few terms on a small grid) to 0.5 s (32 terms on a large one) at
- * the first application; a program that applies a table only a few times may
- * want psb_set_generic_compile(0). Same arithmetic, same results; without
- * NVRTC or the library's device headers (csrc/ beside lib/, or
+ * tables off the TMA path, for the thread-per-point kernel, once a run brings
+ * them to eight applications or to as long as the compiler takes (0.04 s for a
+ * few terms on a small grid, 0.5 s for 32 on a large one).
+ * Same arithmetic, same results; without NVRTC or the library's device headers (csrc/ beside lib/, or
  * $PHYSIS_B200_CSRC) the interpreting kernel runs. */
 psb_status psb_generic_last_compiled(int *compiled);
-/* Run-time compilation of generic tables on (1, the default unless
- * $PHYSIS_B200_GENERIC_COMPILE=0) or off (0). */
+/* Run-time compilation of generic tables off (0) or on, at the first application
+ * of every table (1); $PHYSIS_B200_GENERIC_COMPILE=0 / 1 likewise. The default
+ * is on, with the first few applications off the TMA path interpreted. */
 psb_status psb_set_generic_compile(int on);
 
 /* Compiled stencils: a DSL stencil function (docs/programming.md:117-190 of

@@ -608,7 +608,9 @@ def get_fp_mode():
 
 
 def set_generic_compile(on):
-    """Run-time compilation of generic tables on the TMA path (default on)."""
+    """Run-time compilation of generic tables: off, or on at the first
+    application (the default lets tables off the TMA path be interpreted for
+    their first few)."""
     check(lib.psb_set_generic_compile(1 if on else 0), "psb_set_generic_compile")
 
 

@@ -85,6 +85,10 @@ struct MapImpl {
 struct GenericDesc {
   psb_generic_stencil host;
   void *dev = nullptr;  // device copy of the compact table
+  // Applications so far and their terms over all points, with the current run's;
+  // interpret: too little of either for a compiler run (generic_note_uses).
+  double uses = 0, work = 0;
+  bool interpret = false;
 };
 
 // Kernel launch configuration for the fast paths.
@@ -229,6 +233,9 @@ psb_status generic_tma_launch(MapImpl &m, const GenericDesc &gd, int color, cuda
                               int64_t *launches);
 void generic_note_impl(int impl);
 bool generic_compile_on();
+bool generic_compile_forced();  // by psb_set_generic_compile(1) or the environment
+// A run applies the table `uses` times to `points` points.
+void generic_note_uses(GenericDesc &gd, double uses, double points);
 // The point kernel compiled for the table (k_generic_pt.cu):
 // PSB_ERR_UNSUPPORTED when the map keeps the interpreting kernel.
 psb_status generic_points_launch(MapImpl &m, const GenericDesc &gd, int color, cudaStream_t s,

@@ -5,8 +5,8 @@
 // that the plane pipeline (k_generic_tma.cu) does not take -- red-black
 // order, in-place updates, one- and two-dimensional domains, mixed element
 // types, grids of lower dimension, integer grids, offsets beyond the halo --
-// is compiled here when its map first runs: the term program is written out
-// as straight-line code over the map's strided views, with every factor's
+// is compiled here when its map runs (generic_note_uses says from when on): the
+// term program is written out as straight-line code over the map's strided views, with every factor's
 // grid, type, axes, offset and index form a constant.
 //
 // What bounds it: k_generic (k_generic.cu), which interprets the table,
@@ -201,10 +201,22 @@ std::string key_of(const psb_generic_stencil &d, const GpShape &sh) {
 
 }  // namespace
 
+// The compiler takes 40 ms (four terms, one point a thread) to 540 ms (32 terms,
+// four points a thread: about 40 + 15 a term), interpreting 5 us an application
+// and 14 ps a term and point: a table that is applied a few times is interpreted.
+// It is compiled for the run that brings it to eight applications (a loop; each
+// gains 2.4 to 15 times, from 16^3 up) or to as long as the compiler takes.
+void generic_note_uses(GenericDesc &gd, double uses, double points) {
+  gd.uses += uses;
+  gd.work += uses * points * gd.host.nterms;
+  gd.interpret =
+      !generic_compile_forced() && gd.uses < 8 && gd.work < 1e9 * (3 + gd.host.nterms);
+}
+
 // PSB_ERR_UNSUPPORTED when the map keeps k_generic: a written grid that does
 // not follow the domain's axes one to one, columns near the largest int, no
-// run-time compiler, or a kernel that is not compiled yet while the stream is
-// being captured.
+// run-time compiler, or a kernel that is not compiled yet while the table has
+// been used too little or the stream is being captured.
 psb_status generic_points_launch(MapImpl &m, const GenericDesc &gd, int color, cudaStream_t s,
                                  int64_t *launches) {
   const psb_generic_stencil &d = gd.host;
@@ -278,6 +290,7 @@ psb_status generic_points_launch(MapImpl &m, const GenericDesc &gd, int color, c
   CUfunction fn = nullptr;
   cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
   if (rtc_cached(key, &fn) != PSB_OK) {
+    if (gd.interpret) return PSB_ERR_UNSUPPORTED;
     if (cudaStreamIsCapturing(s, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone)
       return PSB_ERR_UNSUPPORTED;  // no compile or module load here
     if (rtc_function(key, source_of(d, sh), "psb_generic_points", {}, 0, &fn) != PSB_OK)

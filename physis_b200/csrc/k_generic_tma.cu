@@ -96,15 +96,19 @@ static GtFactor gt_compact(const psb_factor &f, const GtPlan &p, int plane_elems
 
 static int g_last_generic_impl = PSB_IMPL_GENERIC;
 static int g_last_generic_compiled = 0;
-static int g_generic_compile = -1;  // -1: $PHYSIS_B200_GENERIC_COMPILE (default on)
+// 0 never, 1 at the first application, 2 (default) the same on the TMA path and
+// after the first few off it; -1: $PHYSIS_B200_GENERIC_COMPILE not read yet.
+static int g_generic_compile = -1;
 
 bool generic_compile_on() {
   if (g_generic_compile < 0) {
     const char *e = getenv("PHYSIS_B200_GENERIC_COMPILE");
-    g_generic_compile = e && e[0] == '0' ? 0 : 1;
+    g_generic_compile = !e || !e[0] ? 2 : e[0] == '0' ? 0 : 1;
   }
-  return g_generic_compile == 1;
+  return g_generic_compile != 0;
 }
+
+bool generic_compile_forced() { return generic_compile_on() && g_generic_compile == 1; }
 
 // Source of a kernel for one table, the library's device headers plus its
 // term program written out with every structural field as a constant.

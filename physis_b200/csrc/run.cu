@@ -37,6 +37,20 @@ static const GenericDesc *generic_of(int kernel_id) {
   return &rt().generics[i];
 }
 
+// The uses that a run makes of its maps' tables.
+static void note_uses(MapImpl **ms, int n, int iter) {
+  for (int i = 0; i < n; i++) {
+    const MapImpl &m = *ms[i];
+    if (!generic_of(m.kernel_id)) continue;
+    GenericDesc &gd = rt().generics[m.kernel_id - PSB_KERNEL_FIRST_GENERIC];
+    double points = 1;
+    for (int k = 0; k < gd.host.ndims; k++)
+      points *= std::max(0, m.dom.local_max[k] - m.dom.local_min[k]);
+    const bool both = m.color == 2;  // two launches, each over half of the points
+    generic_note_uses(gd, (both ? 2.0 : 1.0) * iter, points / (m.color >= 0 ? 2 : 1));
+  }
+}
+
 static const psb_compiled_stencil *compiled_of(int kernel_id) {
   int i = kernel_id - PSB_KERNEL_FIRST_COMPILED;
   if (i < 0 || i >= (int)rt().compiled.size()) return nullptr;
@@ -284,9 +298,13 @@ static psb_status launch_iteration(MapImpl **ms, int n, int64_t *launches) {
 
 static std::string graph_key(MapImpl **ms, int n, int unroll) {
   // Maps are identified by their slot; a slot is only reused after
-  // psb_stencil_free, which drops every cached graph.
+  // psb_stencil_free, which drops every cached graph. A graph of a table that
+  // was still interpreted is not the one of later runs.
   std::string k = std::to_string(unroll) + ":";
-  for (int i = 0; i < n; i++) k += std::to_string(ms[i] - rt().maps.data()) + ",";
+  for (int i = 0; i < n; i++) {
+    const GenericDesc *gd = generic_of(ms[i]->kernel_id);
+    k += std::to_string(ms[i] - rt().maps.data()) + (gd && gd->interpret ? "i," : ",");
+  }
   return k;
 }
 
@@ -483,6 +501,7 @@ static psb_status run_maps(MapImpl **ms, int n, int iter) {
   Runtime &r = rt();
   if (iter <= 0) return PSB_OK;
   for (int i = 0; i < n; i++) PSB_CHECK(check_map(*ms[i]));
+  note_uses(ms, n, iter);
   const bool pipe = r.impl != PSB_IMPL_PLAIN && r.impl != PSB_IMPL_GENERIC && iter >= 2 &&
                     pipe_pair(ms, n);
   for (int i = 0; i < n && !pipe; i++) PSB_CHECK(prepare_ghosts(*ms[i]));
